@@ -17,6 +17,9 @@ CSRC = PACKAGE_DIR / "csrc"
 INCLUDE = PACKAGE_DIR.parent / "include"
 LIBRARY = PACKAGE_DIR / "libstargaze_b200.so"
 
+# Sources compiled once per landscape and FP64-sites variant: one object each,
+# so that they build in parallel. Slowest first.
+VARIANT_SOURCES = ["sg_pixel_kernels.cu", "sg_wave_stages.cu", "sg_wave_adjoint_stages.cu"]
 SOURCES = ["sg_kernels.cu", "sg_wavefront.cu", "sg_wave_adjoint.cu", "sg_display.cu", "sg_host.cpp", "sg_noalloc.cu"]
 HEADERS = ["sg_adjoint.cuh", "sg_device.cuh", "sg_surface.cuh", "sg_integrator.cuh", "sg_air.cuh", "sg_internal.h", "sg_landscape.cuh", "sg_wave_common.cuh"]
 
@@ -41,7 +44,7 @@ def nvcc_path() -> str:
 
 
 def _inputs() -> list[Path]:
-    files = [CSRC / s for s in SOURCES] + [CSRC / h for h in HEADERS]
+    files = [CSRC / s for s in VARIANT_SOURCES + SOURCES] + [CSRC / h for h in HEADERS]
     files.append(INCLUDE / "stargaze_b200.h")
     files.append(Path(__file__))
     return files
@@ -54,9 +57,20 @@ def up_to_date() -> bool:
     return all(p.stat().st_mtime <= built for p in _inputs())
 
 
-def _compile(source: str, objdir: Path) -> tuple[Path, str]:
-    obj = objdir / (Path(source).stem + ".o")
-    cmd = [nvcc_path(), *ARCH_FLAGS, *NVCC_FLAGS, "-c", "-o", str(obj), str(CSRC / source)]
+def _units() -> list[tuple[str, str, list[str]]]:
+    """(source, object name, defines) of every object."""
+    units = []
+    for land in (1, 0):
+        for fp64 in (0, 1):
+            for s in VARIANT_SOURCES:
+                units.append((s, f"{Path(s).stem}_{land}{fp64}.o", [f"-DSG_STAGE_L={land}", f"-DSG_STAGE_F={fp64}"]))
+    return units + [(s, Path(s).stem + ".o", []) for s in SOURCES]
+
+
+def _compile(unit: tuple[str, str, list[str]], objdir: Path) -> tuple[Path, str]:
+    source, name, defines = unit
+    obj = objdir / name
+    cmd = [nvcc_path(), *ARCH_FLAGS, *NVCC_FLAGS, *defines, "-c", "-o", str(obj), str(CSRC / source)]
     proc = subprocess.run(cmd, cwd=str(CSRC), capture_output=True, text=True)
     if proc.returncode != 0:
         raise RuntimeError(f"nvcc failed ({proc.returncode}):\n{' '.join(cmd)}\n{proc.stdout}\n{proc.stderr}")
@@ -65,14 +79,15 @@ def _compile(source: str, objdir: Path) -> tuple[Path, str]:
 
 def build_library(force: bool = False, verbose: bool = False) -> Path:
     """Compile the kernels and the C-ABI host runtime into LIBRARY: one nvcc
-    per translation unit, run concurrently, then one shared-library link."""
+    per object, run concurrently, then one shared-library link."""
     if not force and up_to_date():
         return LIBRARY
     objdir = PACKAGE_DIR / "_build"
     objdir.mkdir(exist_ok=True)
-    workers = max(1, min(len(SOURCES), os.cpu_count() or 1))
+    units = _units()
+    workers = max(1, min(len(units), os.cpu_count() or 1))
     with ThreadPoolExecutor(max_workers=workers) as pool:
-        results = list(pool.map(lambda s: _compile(s, objdir), SOURCES))
+        results = list(pool.map(lambda u: _compile(u, objdir), units))
     tmp = LIBRARY.with_suffix(".so.tmp")
     cmd = [nvcc_path(), *ARCH_FLAGS, "-shared", "-o", str(tmp), *[str(obj) for obj, _ in results]]
     proc = subprocess.run(cmd, cwd=str(CSRC), capture_output=True, text=True)

@@ -182,6 +182,27 @@ struct StageMarks {
     size_t used = 0;
 };
 
+// The stage kernels of one variant: the landscape (L), the FP64 sites (F).
+// `finish` is null where vertex checkpoints are stored (their records need
+// the stages' appends). Instantiated in sg_wave_stages.cu and
+// sg_wave_adjoint_stages.cu, one object per (L, F).
+struct WaveStages {
+    const void *extend, *ring, *surface, *finish;
+};
+template <bool L, bool F>
+WaveStages wave_stages(bool air, bool checkpoints);
+template <bool L, bool F>
+WaveStages adjoint_stages();
+
+// The per-pixel kernels of one variant (sg_pixel_kernels.cu).
+struct PixelKernels {
+    const void *trace[2];  // without and with the host air and the surface styles
+    const void *counted;   // the event-counting integrator
+    const void *adjoint, *segments;
+};
+template <bool L, bool F>
+PixelKernels pixel_kernels();
+
 // What one wavefront dispatch ran.
 struct WaveRun {
     uint32_t iterations = 0;  // stage iterations over all chunks

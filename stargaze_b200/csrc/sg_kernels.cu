@@ -124,37 +124,71 @@ __global__ void __launch_bounds__(256) fma_peak_kernel(float seed, int iters, fl
     if (s == 1234.5678f) out[0] = s;
 }
 
-// cache_terrain_geometry (terrain.wgsl:242-285): node AABBs with curvature
-// and a +-0.02 m margin, curved vertices and normals (12+12-bit packed on
-// grids over 1024 cells). One thread per vertex; the first N threads also
-// write one node each. Strict arithmetic keeps the cache bit-identical to an
-// IEEE evaluation, so traversal decisions match the oracle.
+// cache_terrain_geometry (terrain.wgsl:242-285): node boxes with curvature
+// and a +-0.02 m margin, curved heights and normals (12+12-bit packed on
+// grids over 1024 cells), in the records of t_root and below. Thread i writes
+// node record i, leaf record i and the normal of vertex i. Strict arithmetic
+// keeps the cache bit-identical to an IEEE evaluation, so traversal decisions
+// match the oracle.
+__device__ __forceinline__ float2 cached_range(const float *T, uint32_t cells, float scale, float r, uint32_t index,
+                                               float lo_x, float lo_z, float hi_x, float hi_z) {
+    const float near_x = clampf(0.0f, lo_x, hi_x), near_z = clampf(0.0f, lo_z, hi_z);
+    const float far_x = fmaxf(fabsf(lo_x), fabsf(hi_x)), far_z = fmaxf(fabsf(lo_z), fabsf(hi_z));
+    const float lower = __fsub_rn(__fadd_rn(__fmul_rn(T[t_bounds(cells) + index * 2u], scale),
+                                            t_curvature(far_x, far_z, r)), 0.02f);
+    const float upper = __fadd_rn(__fadd_rn(__fmul_rn(T[t_bounds(cells) + index * 2u + 1u], scale),
+                                            t_curvature(near_x, near_z, r)), 0.02f);
+    return make_float2(lower, upper);
+}
+
 __global__ void __launch_bounds__(256) terrain_cache_kernel(float *T, uint32_t cells, float r) {
     const uint32_t index = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t width = t_width(cells);
     const float scale = t_scale_r(r);
-    if (index < t_nodes(cells)) {
+    if (index == 0u) {
+        const float lo = t_coordinate(0u, cells, scale), hi = t_coordinate(cells, cells, scale);
+        const float2 y = cached_range(T, cells, scale, r, 0u, lo, lo, hi, hi);
+        float *c = T + t_root(cells);
+        c[0] = lo, c[1] = y.x, c[2] = lo, c[3] = hi, c[4] = y.y, c[5] = hi;
+    }
+    if (index < t_inner(cells)) {
         const uint3 node = t_node(index, cells);
-        const float lo_x = t_coordinate(node.x, cells, scale), lo_z = t_coordinate(node.y, cells, scale);
-        const float hi_x = t_coordinate(node.x + node.z, cells, scale), hi_z = t_coordinate(node.y + node.z, cells, scale);
-        const float near_x = clampf(0.0f, lo_x, hi_x), near_z = clampf(0.0f, lo_z, hi_z);
-        const float far_x = fmaxf(fabsf(lo_x), fabsf(hi_x)), far_z = fmaxf(fabsf(lo_z), fabsf(hi_z));
-        const float lower = __fsub_rn(__fadd_rn(__fmul_rn(T[t_bounds(cells) + index * 2u], scale),
-                                                t_curvature(far_x, far_z, r)), 0.02f);
-        const float upper = __fadd_rn(__fadd_rn(__fmul_rn(T[t_bounds(cells) + index * 2u + 1u], scale),
-                                                t_curvature(near_x, near_z, r)), 0.02f);
-        float *c = T + t_cache(cells) + (size_t)index * 6u;
-        c[0] = lo_x;
-        c[1] = lower;
-        c[2] = lo_z;
-        c[3] = hi_x;
-        c[4] = upper;
-        c[5] = hi_z;
+        float x[3], z[3];
+        for (uint32_t k = 0; k < 3u; ++k) {
+            x[k] = t_coordinate(node.x + k * (node.z / 2u), cells, scale);
+            z[k] = t_coordinate(node.y + k * (node.z / 2u), cells, scale);
+        }
+        float2 y[4];
+        for (uint32_t k = 0; k < 4u; ++k) {
+            const uint32_t i = k & 1u, j = k >> 1;
+            y[k] = cached_range(T, cells, scale, r, 4u * index + 1u + k, x[i], z[j], x[i + 1u], z[j + 1u]);
+        }
+        float4 *c = reinterpret_cast<float4 *>(T + t_node_records(cells)) + 4u * (size_t)index;
+        c[0] = make_float4(x[0], x[1], x[2], z[0]);
+        c[1] = make_float4(z[1], z[2], y[0].x, y[0].y);
+        c[2] = make_float4(y[1].x, y[1].y, y[2].x, y[2].y);
+        c[3] = make_float4(y[3].x, y[3].y, 0.0f, 0.0f);
+    }
+    if (index < t_leaves(cells)) {
+        const uint3 node = t_node(t_inner(cells) + index, cells);
+        float x[3], z[3], y[9];
+        for (uint32_t k = 0; k < 3u; ++k) {
+            x[k] = t_coordinate(node.x + k, cells, scale);
+            z[k] = t_coordinate(node.y + k, cells, scale);
+        }
+        for (uint32_t k = 0; k < 9u; ++k) {
+            const uint32_t i = k % 3u, j = k / 3u;
+            y[k] = __fadd_rn(__fmul_rn(T[(node.y + j) * width + node.x + i], scale), t_curvature(x[i], z[j], r));
+        }
+        float4 *c = reinterpret_cast<float4 *>(T + t_leaf_records(cells)) + 4u * (size_t)index;
+        c[0] = make_float4(x[0], x[1], x[2], z[0]);
+        c[1] = make_float4(z[1], z[2], y[0], y[1]);
+        c[2] = make_float4(y[2], y[3], y[4], y[5]);
+        c[3] = make_float4(y[6], y[7], y[8], 0.0f);
     }
     if (index >= t_vertices(cells)) return;
     const uint32_t x = index % width, z = index / width;
     const float px = t_coordinate(x, cells, scale), pz = t_coordinate(z, cells, scale);
-    const float vy = __fadd_rn(__fmul_rn(T[z * width + x], scale), t_curvature(px, pz, r));
     const float denom =
         __fsqrt_rn(fmaxf(__fsub_rn(__fmul_rn(r, r), __fadd_rn(__fmul_rn(px, px), __fmul_rn(pz, pz))), 1.0f));
     const float gx = __fdiv_rn(px, denom), gz = __fdiv_rn(pz, denom);
@@ -172,29 +206,23 @@ __global__ void __launch_bounds__(256) terrain_cache_kernel(float *T, uint32_t c
         normal = f3(__fadd_rn(-T[vertices + index], gx), 1.0f, __fadd_rn(-T[2u * vertices + index], gz));
     }
     normal = mul_rn(normal, __fdiv_rn(1.0f, length_rn(normal)));
-    float *v = T + t_vertex_cache(cells) + (size_t)index * t_vertex_stride(cells);
+    float *v = T + t_normals(cells) + (size_t)index * t_normal_stride(cells);
     if (t_compact(cells)) {
-        v[0] = vy;
         // WGSL round() is round-half-to-even, as rintf.
         const float ux = rintf(__fmul_rn(clampf(__fadd_rn(__fmul_rn(normal.x, 0.5f), 0.5f), 0.0f, 1.0f), 4095.0f));
         const float uz = rintf(__fmul_rn(clampf(__fadd_rn(__fmul_rn(normal.z, 0.5f), 0.5f), 0.0f, 1.0f), 4095.0f));
-        v[1] = (float)((uint32_t)ux | ((uint32_t)uz << 12));
+        v[0] = (float)((uint32_t)ux | ((uint32_t)uz << 12));
     } else {
-        v[0] = px;
-        v[1] = vy;
-        v[2] = pz;
-        v[3] = normal.x;
-        v[4] = normal.y;
-        v[5] = normal.z;
+        v[0] = normal.x;
+        v[1] = normal.y;
+        v[2] = normal.z;
     }
 }
 
 }  // namespace
 
 size_t terrain_source_floats(uint32_t cells) { return (size_t)t_source(cells); }
-size_t terrain_floats(uint32_t cells) {
-    return (size_t)t_vertex_cache(cells) + (size_t)t_vertices(cells) * t_vertex_stride(cells);
-}
+size_t terrain_floats(uint32_t cells) { return t_floats(cells); }
 
 cudaError_t launch_terrain_cache(float *terrain, uint32_t cells, float radius_m, cudaStream_t stream) {
     const uint32_t threads = t_vertices(cells) > t_nodes(cells) ? t_vertices(cells) : t_nodes(cells);

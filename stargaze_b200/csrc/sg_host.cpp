@@ -901,8 +901,11 @@ static int ensure_checkpoints(sg_context *ctx, cudaStream_t stream) {
 }
 
 // Camera rays of frames with at most 32 bodies test only the bodies and
-// rings their 16x16 tile can see: the tile masks, into p.camera_cull.
-static int camera_cull(sg_context *ctx, const sg_frame *frame, sg::TraceParams &p, cudaStream_t stream) {
+// rings their 16x16 tile can see (launch_camera_cull): the buffers of the
+// tile masks and the list of tiles to trace.
+static int ensure_cull(sg_context *ctx, const sg_frame *frame, uint2 **masks, uint32_t **active, cudaStream_t stream) {
+    *masks = nullptr;
+    *active = nullptr;
     if (frame->n_bodies > 32u || frame->n_bodies == 0u) return SG_OK;
     const size_t tiles = (size_t)((ctx->width + 15u) / 16u) * ((ctx->height + 15u) / 16u);
     if (ctx->camera_cull_tiles < tiles) {
@@ -910,13 +913,24 @@ static int camera_cull(sg_context *ctx, const sg_frame *frame, sg::TraceParams &
         cudaFree(ctx->camera_cull);
         ctx->camera_cull = nullptr;
         ctx->camera_cull_tiles = 0;
-        SG_CUDA(ctx, cudaMalloc(&ctx->camera_cull, tiles * sizeof(uint2)));
+        SG_CUDA(ctx, cudaMalloc(&ctx->camera_cull, tiles * (sizeof(uint2) + sizeof(uint32_t))));
         ctx->camera_cull_tiles = tiles;
     }
-    cudaError_t e = sg::launch_camera_cull(p, ctx->camera_cull, stream);
+    *masks = ctx->camera_cull;
+    *active = reinterpret_cast<uint32_t *>(ctx->camera_cull + ctx->camera_cull_tiles);
+    return SG_OK;
+}
+
+// The masks alone, for the per-pixel kernels.
+static int camera_cull(sg_context *ctx, const sg_frame *frame, sg::TraceParams &p, cudaStream_t stream) {
+    uint2 *masks = nullptr;
+    uint32_t *active = nullptr;
+    int status = ensure_cull(ctx, frame, &masks, &active, stream);
+    if (status != SG_OK || !masks) return status;
+    cudaError_t e = sg::launch_camera_cull(p, masks, nullptr, nullptr, false, stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "camera cull masks");
     ctx->launches += 1;
-    p.camera_cull = ctx->camera_cull;
+    p.camera_cull = masks;
     return SG_OK;
 }
 
@@ -962,9 +976,6 @@ static int encode_impl(sg_context *ctx, const sg_frame *frame, void *stream_ptr,
         if (events) {
             SG_CUDA(ctx, cudaMemsetAsync(ctx->events, 0, sg::kEventCount * sizeof(unsigned long long), stream));
             p.events = ctx->events;
-        } else {
-            status = camera_cull(ctx, frame, p, stream);
-            if (status != SG_OK) return status;
         }
         const bool checkpointing = ctx->ck_every > 0u && !events && ctx->integrator == SG_INTEGRATOR_WAVEFRONT &&
                                    !p.air_on && !p.styled && !p.sky_on;
@@ -973,6 +984,7 @@ static int encode_impl(sg_context *ctx, const sg_frame *frame, void *stream_ptr,
         if (!events && ctx->integrator == SG_INTEGRATOR_WAVEFRONT) {
             sg::WaveParams w{};
             status = ensure_wave(ctx, count, w);
+            if (status == SG_OK) status = ensure_cull(ctx, frame, &w.cull, &w.active, stream);
             if (status != SG_OK) return status;
             if (ctx->ck_valid) {
                 status = ensure_checkpoints(ctx, stream);
@@ -1004,6 +1016,10 @@ static int encode_impl(sg_context *ctx, const sg_frame *frame, void *stream_ptr,
                 }
             }
         } else {
+            if (!events) {
+                status = camera_cull(ctx, frame, p, stream);
+                if (status != SG_OK) return status;
+            }
             cudaError_t e = sg::launch_trace(p, events != nullptr, stream);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "trace launch");
             ctx->launches += 1;
@@ -1578,7 +1594,7 @@ int sg_backward(sg_context *ctx, const sg_frame *frame, const sg_tape *tape, con
             a.ck.sample_base = accumulated;
             accumulated += s.counts[2];
             sg::TraceParams p = make_params(ctx, s);
-            status = camera_cull(ctx, frame, p, stream);
+            status = staged ? ensure_cull(ctx, frame, &w.cull, &w.active, stream) : camera_cull(ctx, frame, p, stream);
             if (status != SG_OK) return status;
             if (staged) {
                 sg::WaveRun run;

@@ -68,8 +68,11 @@ struct TraceParams {
 };
 
 // The camera-ray cull masks of every 16x16 tile into `out` (tiles_x *
-// tiles_y entries) for frames of at most 32 bodies.
-cudaError_t launch_camera_cull(const TraceParams &p, uint2 *out, cudaStream_t stream);
+// tiles_y entries) for frames of 1 to 32 bodies. With `active` (as many words,
+// and *count zero), also the list of tiles whose camera rays can meet anything,
+// or of all tiles without `skip_empty`.
+cudaError_t launch_camera_cull(const TraceParams &p, uint2 *out, uint32_t *active, uint32_t *count, bool skip_empty,
+                               cudaStream_t stream);
 
 // Geometry cache of the heightfield (cache_terrain_geometry,
 // terrain.wgsl:242-285) for host radius `radius_m`, in place.
@@ -114,7 +117,7 @@ struct WaveCounters {
 constexpr uint32_t kWaveCounterSets = 8;
 
 // How far the GPU has got through a stage loop: at its start, extend of
-// iteration t writes (paths kept, next sample) to slot t % kProgressSlots of
+// iteration t writes (paths kept, samples left) to slot t % kProgressSlots of
 // a ring in mapped host memory, and the host records done[t % ...] after
 // the iteration. The host enqueues iterations ahead of the one it inspects,
 // so the GPU does not wait for it between iterations.
@@ -165,6 +168,13 @@ struct WaveParams {
     uint32_t tiles_x, tiles_y;
     uint32_t chunk_first;     // first sample of the chunk within the dispatch
     uint32_t chunk_samples;   // samples of the chunk
+    // Buffers of launch_camera_cull (null: frames it does not take): the
+    // masks, and the tiles whose camera rays are traced (null: every tile).
+    // With `skip_empty`, a tile without bodies and rings is not in the list:
+    // its samples are zero.
+    uint2 *cull;
+    uint32_t *active, *active_count;
+    bool skip_empty;
     Checkpoints ck;           // vertex checkpoints of the forward (off: ck.records null)
 };
 

@@ -324,72 +324,173 @@ cudaError_t launch_adjoint(const TraceParams &p, const AdjointParams &a, cudaStr
     return cudaLaunchKernel(fn, grid, dim3(kThreads), args, smem, stream);
 }
 
-// Whether a sphere of radius `rho` at `c` (telescope space, camera at the
-// origin) can meet a ray inside the cone of half-angle `alpha` about the
-// unit direction `axis`: the directions that hit an external sphere form
+// A tile's camera rays: the cone of half-angle alpha about the unit direction
+// `axis` (alpha already carries the 1e-3 rad margin below), and its corners'
+// unnormalised directions (x, y, -1) in order around the tile.
+struct TileCone {
+    double3 axis;
+    double cos_a, sin_a;
+    double cx[4], cy[4];
+    bool valid;  // a cone below 90 degrees, all finite: else every body is kept
+};
+
+__device__ __forceinline__ double dot3(double3 a, double3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+
+// Whether no ray of the tile can meet a sphere of radius `rho` at `c` (telescope
+// space, camera at the origin): the directions that hit an external sphere form
 // the cone of half-angle asin(rho / |c|) about c. Radius and angles carry
 // margins (1e-3 relative, 1e-3 rad) far above the f32 error of the exact
-// intersection tests, so a false here is a certain miss there.
-__device__ __forceinline__ bool cone_meets_sphere(double3 axis, double alpha, double3 c, double rho) {
-    const double dist = sqrt(c.x * c.x + c.y * c.y + c.z * c.z);
-    const double r = rho * (1.0 + 1.0e-3);
-    if (!(dist > r)) return true;  // the camera is inside or at the sphere (or the input is not finite)
-    const double cosb = fmin(fmax((axis.x * c.x + axis.y * c.y + axis.z * c.z) / dist, -1.0), 1.0);
-    return acos(cosb) <= alpha + asin(r / dist) + 1.0e-3;
+// intersection tests, so a true here is a certain miss there. With the camera
+// within the margin of the surface (an observer on the ground), the tile is
+// culled only when the exact test's own f32 value of |c|^2 - r^2, the same for
+// every camera ray, is positive (`outside`) and every ray points more than
+// 90 degrees and the margin away from the centre: that test's early out.
+__device__ __forceinline__ bool cone_misses_sphere(const TileCone &t, double3 c, double rho, bool outside) {
+    const double dist = sqrt(dot3(c, c)), r = rho * (1.0 + 1.0e-3);
+    const double cos_g = dot3(t.axis, c) / dist;
+    if (!(dist > r)) return outside && cos_g < -t.sin_a;
+    const double sin_b = r / dist, cos_b = sqrt(1.0 - sin_b * sin_b);
+    return t.sin_a * cos_b + t.cos_a * sin_b > 0.0 && cos_g < t.cos_a * cos_b - t.sin_a * sin_b;
 }
 
-__device__ __forceinline__ double3 unit_direction(double ndc_x, double ndc_y, double tangent, double aspect) {
-    const double x = ndc_x * tangent * aspect, y = ndc_y * tangent;
-    const double inv = 1.0 / sqrt(x * x + y * y + 1.0);
-    return make_double3(x * inv, y * inv, -inv);
+// Whether no ray of the tile can cross the annulus [inner, outer] about c in
+// the plane of normal n. A tile whose rays all cross the plane on one side of
+// the camera maps to a convex quadrilateral of the plane: its radii lie between
+// its distance from c and its farthest corner's. Margins: 1e-3 of the radii
+// and 1e-4 of the centre's distance, over plane angles above 0.01, where the
+// f32 error of the exact test's crossing is below 1e-4 of that distance.
+__device__ __forceinline__ bool tile_misses_annulus(const TileCone &t, double3 c, double3 n, double inner, double outer) {
+    const double nn = dot3(n, n);
+    if (!(nn > 0.0)) return false;
+    const double scale = 1.0 / sqrt(nn);
+    n = make_double3(n.x * scale, n.y * scale, n.z * scale);
+    const double h = dot3(n, c), dist = sqrt(dot3(c, c)), slack = 1.0e-4 * dist;
+    double den[4], longest = 0.0, steepest = 1.0e300;
+    bool positive = true, negative = true;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        den[k] = n.x * t.cx[k] + n.y * t.cy[k] - n.z;
+        longest = fmax(longest, t.cx[k] * t.cx[k] + t.cy[k] * t.cy[k] + 1.0);
+        steepest = fmin(steepest, fabs(den[k]));
+        positive = positive && den[k] > 0.0;
+        negative = negative && den[k] < 0.0;
+    }
+    if (!(positive || negative) || !(steepest > 0.01 * sqrt(longest))) return false;
+    double3 p[4];
+    double farthest = 0.0;
+    bool behind = true, ahead = true;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double s = h / den[k];
+        const double along = s * sqrt(t.cx[k] * t.cx[k] + t.cy[k] * t.cy[k] + 1.0);
+        behind = behind && along < -1.0e-3 * dist;
+        ahead = ahead && s > 0.0;
+        p[k] = make_double3(s * t.cx[k] - c.x, s * t.cy[k] - c.y, -s - c.z);
+        farthest = fmax(farthest, dot3(p[k], p[k]));
+    }
+    if (behind) return true;
+    if (!ahead) return false;
+    if (sqrt(farthest) < inner * (1.0 - 1.0e-3) - slack) return true;
+    double nearest = 1.0e300;
+    bool left = true, right = true;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double3 a = p[k], b = p[(k + 1) & 3];
+        const double3 e = make_double3(b.x - a.x, b.y - a.y, b.z - a.z);
+        const double w = n.x * (a.y * b.z - a.z * b.y) + n.y * (a.z * b.x - a.x * b.z) + n.z * (a.x * b.y - a.y * b.x);
+        left = left && w >= 0.0;
+        right = right && w <= 0.0;
+        const double u = fmin(fmax(-dot3(a, e) / fmax(dot3(e, e), 1.0e-300), 0.0), 1.0);
+        const double3 q = make_double3(a.x + u * e.x, a.y + u * e.y, a.z + u * e.z);
+        nearest = fmin(nearest, dot3(q, q));
+    }
+    return !left && !right && sqrt(nearest) > outer * (1.0 + 1.0e-3) + slack;
 }
 
-// One CTA per 16x16 tile, one thread per body: the bodies (their point
-// discs included) and the rings a camera ray of the tile may meet. A camera
-// ray of pixel (x, y) has ndc in [2x/W - 1, 2(x+1)/W - 1] x [1 - 2(y+1)/H,
-// 1 - 2y/H] (camera_direction, pathtrace.wgsl:1619-1626); the tile's rays
-// lie in the cone about its centre ray through its farthest corner.
-__global__ void __launch_bounds__(32) camera_cull_kernel(const __grid_constant__ TraceParams P, uint2 *out,
-                                                         uint32_t tiles_x) {
-    const uint32_t tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
-    const uint32_t i = threadIdx.x;
+// `group` lanes per 16x16 tile, one per body (the power of two at or above
+// their number): the bodies (their point discs included) and the rings a
+// camera ray of the tile may meet. A camera ray of pixel (x, y) has ndc in
+// [2x/W - 1, 2(x+1)/W - 1] x [1 - 2(y+1)/H, 1 - 2y/H] (camera_direction,
+// pathtrace.wgsl:1619-1626); the tile's rays lie in the cone about its centre
+// ray through its farthest corner. With `active`, the tiles that can meet
+// anything (every tile, without `skip_empty`) are appended to it, their number
+// added to *count (zero before the launch); tiles of one warp keep their order.
+__global__ void __launch_bounds__(128) camera_cull_kernel(const __grid_constant__ TraceParams P, uint2 *out,
+                                                          uint32_t *active, uint32_t *count, bool skip_empty,
+                                                          uint32_t group, uint32_t tiles_x, uint32_t tiles) {
+    const uint32_t thread = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    const uint32_t tile = thread / group, i = thread % group;
     const uint32_t n = P.s.counts[0];
     bool body = false, ring = false;
-    if (i < n) {
+    if (tile < tiles && i < n) {
+        const uint32_t tx = tile % tiles_x, ty = tile / tiles_x;
         const double w = P.s.g.viewport[0], h = P.s.g.viewport[1];
         const double tangent = P.s.g.cam_forward[3], aspect = P.s.g.viewport[3];
-        const double x0 = 2.0 * (tx * kTile) / w - 1.0, x1 = 2.0 * fmin((double)(tx * kTile + kTile), w) / w - 1.0;
-        const double y0 = 1.0 - 2.0 * fmin((double)(ty * kTile + kTile), h) / h, y1 = 1.0 - 2.0 * (ty * kTile) / h;
-        const double3 axis = unit_direction(0.5 * (x0 + x1), 0.5 * (y0 + y1), tangent, aspect);
-        double alpha = 0.0;
-        const double cx[2] = {x0, x1}, cy[2] = {y0, y1};
-        for (int a = 0; a < 2; ++a)
-            for (int b = 0; b < 2; ++b) {
-                const double3 d = unit_direction(cx[a], cy[b], tangent, aspect);
-                const double c = fmin(fmax(d.x * axis.x + d.y * axis.y + d.z * axis.z, -1.0), 1.0);
-                alpha = fmax(alpha, acos(c));
-            }
+        const double x0 = (2.0 * (tx * kTile) / w - 1.0) * tangent * aspect;
+        const double x1 = (2.0 * fmin((double)(tx * kTile + kTile), w) / w - 1.0) * tangent * aspect;
+        const double y0 = (1.0 - 2.0 * fmin((double)(ty * kTile + kTile), h) / h) * tangent;
+        const double y1 = (1.0 - 2.0 * (ty * kTile) / h) * tangent;
+        TileCone t;
+        t.cx[0] = x0, t.cx[1] = x1, t.cx[2] = x1, t.cx[3] = x0;
+        t.cy[0] = y0, t.cy[1] = y0, t.cy[2] = y1, t.cy[3] = y1;
+        const double ax = 0.5 * (x0 + x1), ay = 0.5 * (y0 + y1), al = 1.0 / sqrt(ax * ax + ay * ay + 1.0);
+        t.axis = make_double3(ax * al, ay * al, -al);
+        double c = 1.0;
+        t.valid = true;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const double v = (t.cx[k] * t.axis.x + t.cy[k] * t.axis.y - t.axis.z) /
+                             sqrt(t.cx[k] * t.cx[k] + t.cy[k] * t.cy[k] + 1.0);
+            t.valid = t.valid && v > 0.0 && v < 1.0 + 1.0e-9;
+            c = fmin(c, v);
+        }
+        // alpha + 1e-3 rad.
+        const double s = sqrt(fmax(1.0 - c * c, 0.0));
+        constexpr double kMarginCos = 0.9999995000000417, kMarginSin = 9.999998333333417e-4;
+        t.cos_a = c * kMarginCos - s * kMarginSin;
+        t.sin_a = s * kMarginCos + c * kMarginSin;
         const float4 hi = P.bodies[i * kBodyVec4 + kCenter], lo = P.bodies[i * kBodyVec4 + kLow];
-        const double3 c = make_double3((double)hi.x + lo.x, (double)hi.y + lo.y, (double)hi.z + lo.z);
-        const double dist = sqrt(c.x * c.x + c.y * c.y + c.z * c.z);
+        const double3 centre = make_double3((double)hi.x + lo.x, (double)hi.y + lo.y, (double)hi.z + lo.z);
+        const double dist = sqrt(dot3(centre, centre));
         // point_disc_hit draws an unresolved body as a disc of at least
         // `angle` radians (pathtrace.wgsl:1308-1333).
         const double pixel = 2.0 * tangent / fmax(h, 1.0);
         const double angle = fmin(fmax((double)kPointDiscRadius, 0.7 * pixel), (double)kStarDotPixels * pixel);
-        const double radius = hi.w;
-        body = cone_meets_sphere(axis, alpha, c, fmax(radius, angle * dist));
+        const double radius = hi.w, drawn = fmax(radius, angle * dist);
+        const float3 oc = add_rn(xyz(hi), xyz(lo));  // relative_center of a camera ray
+        const bool outside = drawn == radius && __fsub_rn(dot_rn(oc, oc), __fmul_rn(hi.w, hi.w)) > 0.0f;
+        body = !(t.valid && cone_misses_sphere(t, centre, drawn, outside));
         const float4 plane = P.bodies[i * kBodyVec4 + kRingPlane], params = P.bodies[i * kBodyVec4 + kRingParams];
         // The annulus lies inside the sphere of its outer radius.
-        if (params.x > plane.w && params.y > 0.0f) ring = cone_meets_sphere(axis, alpha, c, (double)params.x * radius);
+        if (params.x > plane.w && params.y > 0.0f)
+            ring = !(t.valid && (cone_misses_sphere(t, centre, (double)params.x * radius, false) ||
+                                 tile_misses_annulus(t, centre, make_double3(plane.x, plane.y, plane.z),
+                                                     (double)plane.w * radius, (double)params.x * radius)));
     }
-    const uint32_t bodies = __ballot_sync(0xffffffffu, body), rings = __ballot_sync(0xffffffffu, ring);
-    if (i == 0) out[blockIdx.x] = make_uint2(bodies, rings);
+    const uint32_t shift = lane & ~(group - 1u), field = group == 32u ? 0xffffffffu : (1u << group) - 1u;
+    const uint32_t bodies = (__ballot_sync(0xffffffffu, body) >> shift) & field;
+    const uint32_t rings = (__ballot_sync(0xffffffffu, ring) >> shift) & field;
+    const bool leader = i == 0u && tile < tiles;
+    if (leader) out[tile] = make_uint2(bodies, rings);
+    if (!active) return;
+    const bool taken = leader && (!skip_empty || (bodies | rings) != 0u);
+    const uint32_t taken_lanes = __ballot_sync(0xffffffffu, taken);
+    uint32_t at = 0u;
+    if (lane == 0u && taken_lanes) at = atomicAdd(count, __popc(taken_lanes));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (taken) active[at + __popc(taken_lanes & ((1u << lane) - 1u))] = tile;
 }
 
-cudaError_t launch_camera_cull(const TraceParams &p, uint2 *out, cudaStream_t stream) {
-    const uint32_t tiles_x = (p.width + kTile - 1) / kTile, tiles_y = (p.height + kTile - 1) / kTile;
-    if (p.s.counts[0] > 32u || tiles_x * tiles_y == 0) return cudaErrorInvalidValue;
-    camera_cull_kernel<<<tiles_x * tiles_y, 32, 0, stream>>>(p, out, tiles_x);
+cudaError_t launch_camera_cull(const TraceParams &p, uint2 *out, uint32_t *active, uint32_t *count, bool skip_empty,
+                               cudaStream_t stream) {
+    const uint32_t tiles_x = (p.width + kTile - 1) / kTile, tiles = tiles_x * ((p.height + kTile - 1) / kTile);
+    const uint32_t n = p.s.counts[0];
+    if (n == 0u || n > 32u || tiles == 0u) return cudaErrorInvalidValue;
+    uint32_t group = 1u;
+    while (group < n) group *= 2u;
+    const uint64_t threads = (uint64_t)tiles * group;
+    camera_cull_kernel<<<(uint32_t)((threads + 127u) / 128u), 128, 0, stream>>>(p, out, active, count, skip_empty, group,
+                                                                                tiles_x, tiles);
     return cudaGetLastError();
 }
 

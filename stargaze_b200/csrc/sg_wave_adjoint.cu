@@ -64,7 +64,9 @@ cudaError_t launch_adjoint_wavefront(const TraceParams &params, const AdjointPar
     // iteration bound; see launch_wavefront for the host-side guard.
     const uint64_t cap = 2ull * ((uint64_t)p.s.counts[3] * (p.s.counts[0] + 2u) + 2u);
     const uint64_t bound = ((uint64_t)samples + 1u) * cap;
-    cudaError_t e = cudaMemsetAsync(w.counters, 0, kWaveCounterSets * sizeof(WaveCounters), stream);
+    // A tile whose camera rays meet nothing has no gradient.
+    w.skip_empty = !land;
+    cudaError_t e = cull_tiles(p, w, stream, run);
     if (e != cudaSuccess) return e;
     for (uint64_t t = 0;; ++t) {
         if (t >= bound) return cudaErrorLaunchTimeout;
@@ -81,10 +83,10 @@ cudaError_t launch_adjoint_wavefront(const TraceParams &params, const AdjointPar
         if (t < kLookahead) continue;
         WaveStart start;
         if ((e = started(progress, t - kLookahead, &start)) != cudaSuccess) return e;
-        if (start.kept == 0u && start.next >= samples) break;
+        if (start.kept == 0u && start.left == 0u) break;
         // Every sample is out and few paths are left: no later iteration
         // holds more than iteration t - kLookahead did; finish them at once.
-        if (start.next >= samples && start.kept <= kFinishPaths) {
+        if (start.left == 0u && start.kept <= kFinishPaths) {
             const uint32_t blocks = std::min<uint32_t>(grid[3], (start.kept + kShadeThreads - 1) / kShadeThreads);
             uint32_t next_t = it + 1u;
             if (blocks > 0u) {

@@ -241,8 +241,14 @@ __device__ __forceinline__ WaveCounters *counters(const WaveParams &W, uint32_t 
     return W.counters + (t % kWaveCounterSets);
 }
 
-// Samples of a chunk are numbered sample-major over the padded tile grid.
-__device__ __forceinline__ uint32_t padded_pixels(const WaveParams &W) { return W.tiles_x * W.tiles_y * 256u; }
+// Samples of a chunk are numbered sample-major over the padded pixels of the
+// tiles traced.
+__device__ __forceinline__ uint32_t padded_pixels(const WaveParams &W) {
+    return (W.active ? *W.active_count : W.tiles_x * W.tiles_y) * 256u;
+}
+__device__ __forceinline__ uint32_t camera_tile(const WaveParams &W, uint32_t k) {
+    return W.active ? W.active[k] : k;
+}
 
 // Grid of a persistent stage kernel: every resident CTA slot of every SM.
 // (Asking for the largest L1 share through the shared-memory carveout
@@ -266,26 +272,35 @@ inline cudaError_t iteration_done(WaveProgress &pr, uint64_t t, cudaStream_t str
     return cudaEventRecord(pr.done[t % kProgressSlots], stream);
 }
 
-// What iteration s started from: the paths kept and the next sample.
+// What iteration s started from: the paths kept and the samples left.
 struct WaveStart {
-    uint32_t kept, next;
+    uint32_t kept, left;
 };
 inline cudaError_t started(const WaveProgress &pr, uint64_t s, WaveStart *out) {
     cudaError_t e = cudaEventSynchronize(pr.done[s % kProgressSlots]);
     if (e != cudaSuccess) return e;
     const volatile uint2 *h = pr.host + s % kProgressSlots;
     out->kept = h->x;
-    out->next = h->y;
+    out->left = h->y;
     return cudaSuccess;
 }
 
-// Whether iteration s started with no path kept and no sample left (of
-// `samples`): then it and every later iteration had nothing to do.
-inline cudaError_t drained(const WaveProgress &pr, uint64_t s, uint32_t samples, bool *empty) {
-    WaveStart start;
-    cudaError_t e = started(pr, s, &start);
-    if (e == cudaSuccess) *empty = start.kept == 0u && start.next >= samples;
-    return e;
+// Clears the iteration counters and the active-tile count, and culls the
+// camera rays' tiles: fills w.active_count and p.camera_cull, or clears
+// w.active and w.skip_empty where the frame is not culled.
+inline cudaError_t cull_tiles(TraceParams &p, WaveParams &w, cudaStream_t stream, WaveRun *run) {
+    cudaError_t e = cudaMemsetAsync(w.counters, 0, (kWaveCounterSets + 1u) * sizeof(WaveCounters), stream);
+    if (e != cudaSuccess) return e;
+    if (!w.cull) {
+        w.active = nullptr;
+        w.skip_empty = false;
+        return cudaSuccess;
+    }
+    w.active_count = &w.counters[kWaveCounterSets].cont;
+    if ((e = launch_camera_cull(p, w.cull, w.active, w.active_count, w.skip_empty, stream)) != cudaSuccess) return e;
+    p.camera_cull = w.cull;
+    run->kernels += 1;
+    return cudaSuccess;
 }
 
 inline cudaError_t mark(StageMarks *m, int stage, cudaStream_t stream) {

@@ -41,12 +41,13 @@ __global__ void __launch_bounds__(kThreads, SG_WAVE_EXTEND_MIN_BLOCKS) wave_exte
     // chunk fill the pool up to n.
     const uint32_t kept = c->cont, next = c->next;
     const uint32_t per_sample = padded_pixels(W);
-    const uint32_t take = min(W.pool - kept, per_sample * W.chunk_samples - next);
+    const uint32_t left = per_sample * W.chunk_samples - next;
+    const uint32_t take = min(W.pool - kept, left);
     const uint32_t n = kept + take;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         counters(W, t + 1u)->next = next + take;
         *counters(W, t + 2u) = WaveCounters{};
-        W.progress[t % kProgressSlots] = make_uint2(kept, next);
+        W.progress[t % kProgressSlots] = make_uint2(kept, left);
     }
     if (blockIdx.x * kThreads * kItems >= n) return;
     const Scene S = stage_scene(P, smem);
@@ -75,7 +76,7 @@ __global__ void __launch_bounds__(kThreads, SG_WAVE_EXTEND_MIN_BLOCKS) wave_exte
                 const uint32_t k = next + (i - kept);
                 const uint32_t smp = k / per_sample;
                 const uint32_t q = k - smp * per_sample;
-                const uint32_t tile = q >> 8, within = q & 255u;
+                const uint32_t tile = camera_tile(W, q >> 8), within = q & 255u;
                 const uint32_t warp = within >> 5, lane = within & 31u;
                 const uint32_t x = (tile % W.tiles_x) * kTile + (warp & 1u) * 8u + (lane & 7u);
                 const uint32_t y = (tile / W.tiles_x) * kTile + (warp >> 1) * 4u + (lane >> 3);

@@ -45,7 +45,13 @@ __global__ void __launch_bounds__(kThreads) wave_resolve(const __grid_constant__
     const uint32_t pixel = blockIdx.x * kThreads + threadIdx.x;
     if (pixel >= pixels) return;
     float4 total = first ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : W.totals[pixel];
-    for (uint32_t smp = 0; smp < W.chunk_samples; ++smp) {
+    // The samples of a tile that is not traced are zero.
+    uint32_t samples = W.chunk_samples;
+    if (W.skip_empty) {
+        const uint2 m = P.camera_cull[(pixel / P.width / kTile) * W.tiles_x + pixel % P.width / kTile];
+        if ((m.x | m.y) == 0u) samples = 0u;
+    }
+    for (uint32_t smp = 0; smp < samples; ++smp) {
         const float4 r = W.results[(size_t)smp * pixels + pixel];
         total.x += r.x;
         total.y += r.y;
@@ -112,7 +118,7 @@ cudaError_t run_iteration(const WaveStages &stages, TraceParams &p, WaveParams &
 
 size_t wave_state_bytes(uint32_t pool) {
     return (size_t)pool * sizeof(float4) * (2 * kWavePlanes + kWaveHitPlanes) + (size_t)pool * 2 * sizeof(uint32_t) +
-           kWaveCounterSets * sizeof(WaveCounters);
+           (kWaveCounterSets + 1u) * sizeof(WaveCounters);
 }
 
 size_t wave_result_bytes(uint32_t pixels, uint32_t chunk_samples) {
@@ -151,6 +157,10 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
     w.tiles_x = (p.width + kTile - 1) / kTile;
     w.tiles_y = (p.height + kTile - 1) / kTile;
     const uint32_t chunk = w.chunk_samples;
+    // A tile whose camera rays meet no body and no ring needs no paths where a
+    // ray that escapes leaves nothing: no landscape, air, sky or stored totals.
+    w.skip_empty = !land && !air && !p.sky_on && !w.ck.totals;
+    if (cudaError_t e = cull_tiles(p, w, stream, run); e != cudaSuccess) return e;
     const uint32_t per_sample = w.tiles_x * w.tiles_y * 256u;
     // A path ends within max_vertices * (bodies + 2) + 1 iterations, and an
     // iteration that takes no new sample has a full pool of paths that all
@@ -162,7 +172,9 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
         w.chunk_samples = std::min(chunk, z - first);
         const uint32_t samples = per_sample * w.chunk_samples;
         const uint64_t bound = ((uint64_t)samples + 1u) * cap;
-        cudaError_t e = cudaMemsetAsync(w.counters, 0, kWaveCounterSets * sizeof(WaveCounters), stream);
+        // (The first chunk's were cleared with the active-tile count.)
+        cudaError_t e = cudaSuccess;
+        if (first > 0u) e = cudaMemsetAsync(w.counters, 0, kWaveCounterSets * sizeof(WaveCounters), stream);
         if (e != cudaSuccess) return e;
         // The host reads the start of iteration t - kLookahead while the
         // GPU runs the later ones; once one started empty the chunk has
@@ -178,10 +190,10 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
             if (t < kLookahead) continue;
             WaveStart start;
             if ((e = started(progress, t - kLookahead, &start)) != cudaSuccess) return e;
-            if (start.kept == 0u && start.next >= samples) break;
+            if (start.kept == 0u && start.left == 0u) break;
             // Every sample is out and few paths are left: no later iteration
             // holds more than iteration t - kLookahead did; finish them at once.
-            if (set.finish && start.next >= samples && start.kept <= kFinishPaths) {
+            if (set.finish && start.left == 0u && start.kept <= kFinishPaths) {
                 const uint32_t blocks = std::min<uint32_t>(grid[3], (start.kept + kThreads - 1) / kThreads);
                 if (blocks > 0u) {
                     if ((e = mark(marks, kStageFinish, stream)) != cudaSuccess) return e;

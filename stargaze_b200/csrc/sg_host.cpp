@@ -129,6 +129,8 @@ struct sg_context {
     float4 *ck_totals = nullptr;
     size_t ck_totals_size = 0;
     uint32_t *ck_count = nullptr;
+    cudaEvent_t encoded = nullptr;          // the end of the last encode, and its stream
+    cudaStream_t encode_stream = nullptr;
     bool ck_valid = false;                  // every sample so far went through the checkpointing forward
     uint2 *camera_cull = nullptr;           // per-tile cull masks of camera rays
     size_t camera_cull_tiles = 0;
@@ -163,6 +165,20 @@ struct DeviceGuard {
         if (previous >= 0) cudaSetDevice(previous);
     }
 };
+
+// Work on `stream` comes after the last encode, also when that was on another
+// stream (encode returns with its kernels in flight).
+int follow_encode(sg_context *ctx, cudaStream_t stream) {
+    if (ctx->encoded && ctx->encode_stream != stream) SG_CUDA(ctx, cudaStreamWaitEvent(stream, ctx->encoded, 0));
+    return SG_OK;
+}
+
+int mark_encode(sg_context *ctx, cudaStream_t stream) {
+    if (!ctx->encoded) SG_CUDA(ctx, cudaEventCreateWithFlags(&ctx->encoded, cudaEventDisableTiming));
+    SG_CUDA(ctx, cudaEventRecord(ctx->encoded, stream));
+    ctx->encode_stream = stream;
+    return SG_OK;
+}
 
 void free_image(sg_context *ctx) {
     cudaFree(ctx->mean);
@@ -541,6 +557,7 @@ int sg_destroy(sg_context *ctx) {
     for (cudaEvent_t e : ctx->wave_progress.done)
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->stage_marks.events) cudaEventDestroy(e);
+    if (ctx->encoded) cudaEventDestroy(ctx->encoded);
     delete ctx;
     return SG_OK;
 }
@@ -853,6 +870,7 @@ static int meter_exposure(sg_context *ctx, cudaStream_t stream) {
     }
     if (ctx->width == 0 || ctx->height == 0) return SG_OK;
     DeviceGuard guard(ctx->device);
+    if (int status = follow_encode(ctx, stream); status != SG_OK) return status;
     if (!ctx->exposure) SG_CUDA(ctx, cudaMalloc(&ctx->exposure, sizeof(sg::ExposureState)));
     if (!ctx->histogram) SG_CUDA(ctx, cudaMalloc(&ctx->histogram, sg::kExposureBins * sizeof(uint32_t)));
     // Pageable source: the bytes are staged before the call returns.
@@ -931,7 +949,7 @@ static int camera_cull(sg_context *ctx, const sg_frame *frame, sg::TraceParams &
     uint32_t *active = nullptr;
     int status = ensure_cull(ctx, frame, &masks, &active, stream);
     if (status != SG_OK || !masks) return status;
-    cudaError_t e = sg::launch_camera_cull(p, masks, nullptr, nullptr, false, stream);
+    cudaError_t e = sg::launch_camera_cull(p, masks, nullptr, nullptr, false, false, stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "camera cull masks");
     ctx->launches += 1;
     p.camera_cull = masks;
@@ -953,7 +971,8 @@ static int encode_impl(sg_context *ctx, const sg_frame *frame, void *stream_ptr,
     if (count > 0 && ctx->width > 0 && ctx->height > 0) {
         DeviceGuard guard(ctx->device);
         const sg_settings s = pack_settings(ctx, frame, count);
-        status = upload_bodies(ctx, frame, stream);
+        status = follow_encode(ctx, stream);
+        if (status == SG_OK) status = upload_bodies(ctx, frame, stream);
         if (status != SG_OK) return status;
         sg::TraceParams p = make_params(ctx, s);
         for (uint32_t k = 0; k < frame->n_bodies; ++k)
@@ -1038,6 +1057,11 @@ static int encode_impl(sg_context *ctx, const sg_frame *frame, void *stream_ptr,
     }
     status = meter_exposure(ctx, stream);
     if (status != SG_OK) return status;
+    {
+        DeviceGuard guard(ctx->device);
+        status = mark_encode(ctx, stream);
+        if (status != SG_OK) return status;
+    }
     ctx->history.samples += count;
     ctx->history.sequence += count;
     ctx->exposure_idle_frames = count > 0 ? 0u : (ctx->exposure_idle_frames == UINT32_MAX ? UINT32_MAX : ctx->exposure_idle_frames + 1u);
@@ -1111,6 +1135,7 @@ static int read_image(sg_context *ctx, const float4 *src, float *dst, int on_dev
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     const size_t bytes = (size_t)ctx->width * ctx->height * sizeof(float4);
     if (bytes == 0) return SG_OK;
+    if (int status = follow_encode(ctx, stream); status != SG_OK) return status;
     SG_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                                  stream));
     SG_CUDA(ctx, cudaStreamSynchronize(stream));
@@ -1133,6 +1158,7 @@ int sg_set_accumulation(sg_context *ctx, const float *src, int src_on_device, ui
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     const size_t n = (size_t)ctx->width * ctx->height;
     if (n == 0) return SG_OK;
+    if (int status = follow_encode(ctx, stream); status != SG_OK) return status;
     std::vector<float> host(n * 4);
     if (src_on_device) {
         SG_CUDA(ctx, cudaMemcpyAsync(host.data(), src, n * sizeof(float4), cudaMemcpyDeviceToHost, stream));
@@ -1170,6 +1196,7 @@ int sg_upload_ring_profile(sg_context *ctx, uint32_t slot, const float *tau, uin
         if (!(tau[k] >= 0.0f) || !std::isfinite(tau[k]))
             return fail(ctx, SG_ERR_INVALID, "ring optical depths must be finite and non-negative");
     DeviceGuard guard(ctx->device);
+    if (ctx->encoded) SG_CUDA(ctx, cudaEventSynchronize(ctx->encoded));  // a dispatch in flight reads the tables
     if (bins)
         SG_CUDA(ctx, cudaMemcpy(ctx->ring_tables + (size_t)slot * SG_RING_TABLE_MAX_BINS, tau, bins * sizeof(float),
                                 cudaMemcpyHostToDevice));
@@ -1184,7 +1211,8 @@ static int probe_setup(sg_context *ctx, const sg_frame *frame, cudaStream_t stre
     int status = validate_frame(ctx, frame);
     if (status != SG_OK) return status;
     const sg_settings s = pack_settings(ctx, frame, 0);
-    status = upload_bodies(ctx, frame, stream);
+    status = follow_encode(ctx, stream);
+    if (status == SG_OK) status = upload_bodies(ctx, frame, stream);
     if (status != SG_OK) return status;
     *p = make_params(ctx, s);
     return SG_OK;
@@ -1354,11 +1382,12 @@ int sg_display(sg_context *ctx, uint32_t width, uint32_t height, int format, voi
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     const size_t bytes = (size_t)width * height * (format == SG_DISPLAY_RGBA32F ? 16u : 4u);
     void *dst = out;
-    if (!on_device) {
-        int status = ensure_scratch(ctx, bytes);
-        if (status != SG_OK) return status;
+    int status = follow_encode(ctx, stream);
+    if (status == SG_OK && !on_device) {
+        status = ensure_scratch(ctx, bytes);
         dst = ctx->scratch;
     }
+    if (status != SG_OK) return status;
     sg::DisplayParams d{};
     d.mean = ctx->mean;
     d.backdrop = ctx->backdrop;
@@ -1399,6 +1428,7 @@ int sg_get_exposure(sg_context *ctx, float *exposure, void *stream_ptr) {
     }
     DeviceGuard guard(ctx->device);
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+    if (int status = follow_encode(ctx, stream); status != SG_OK) return status;
     float value = 0.0f;
     SG_CUDA(ctx, cudaMemcpyAsync(&value, ctx->exposure, sizeof(float), cudaMemcpyDeviceToHost, stream));
     SG_CUDA(ctx, cudaStreamSynchronize(stream));
@@ -1455,6 +1485,7 @@ int sg_get_checkpoint_stats(sg_context *ctx, uint64_t *device_bytes, uint64_t *r
     uint32_t claimed = 0;
     if (ctx->ck_count) {
         DeviceGuard guard(ctx->device);
+        if (ctx->encoded) SG_CUDA(ctx, cudaEventSynchronize(ctx->encoded));
         SG_CUDA(ctx, cudaMemcpy(&claimed, ctx->ck_count, sizeof(claimed), cudaMemcpyDeviceToHost));
     }
     const uint64_t stored = std::min<uint64_t>(claimed, ctx->ck_capacity);
@@ -1516,6 +1547,8 @@ int sg_backward(sg_context *ctx, const sg_frame *frame, const sg_tape *tape, con
     if (pixels == 0) return SG_OK;
     DeviceGuard guard(ctx->device);
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+    status = follow_encode(ctx, stream);
+    if (status != SG_OK) return status;
     const size_t texels = ctx->albedo_map ? (size_t)ctx->map_width * ctx->map_height : 0;
     const size_t floats = sg::kGradMap + texels;
     if (ctx->grad_floats < floats) {
@@ -1587,8 +1620,6 @@ int sg_backward(sg_context *ctx, const sg_frame *frame, const sg_tape *tape, con
             largest = std::max(largest, std::min<uint32_t>(SG_MAX_BATCH_SAMPLES, tape->count[k]));
         status = ensure_adjoint(ctx, largest, w, x);
         if (status != SG_OK) return status;
-        cudaError_t e = sg::reset_adjoint_slots(x, w.pool, stream);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "adjoint slot reset");
     }
     uint32_t accumulated = 0;  // accumulation index of the launch's first sample
     for (uint32_t k = 0; k < tape->n_ranges; ++k) {

@@ -71,8 +71,9 @@ struct TraceParams {
 // tiles_y entries) for frames of 1 to 32 bodies. With `active` (as many words,
 // and *count zero), also the list of tiles whose camera rays can meet anything,
 // or of all tiles without `skip_empty`.
+// `ordered`: in raster order (one more launch).
 cudaError_t launch_camera_cull(const TraceParams &p, uint2 *out, uint32_t *active, uint32_t *count, bool skip_empty,
-                               cudaStream_t stream);
+                               bool ordered, cudaStream_t stream);
 
 // Geometry cache of the heightfield (cache_terrain_geometry,
 // terrain.wgsl:242-285) for host radius `radius_m`, in place.
@@ -168,6 +169,7 @@ struct WaveParams {
     uint32_t tiles_x, tiles_y;
     uint32_t chunk_first;     // first sample of the chunk within the dispatch
     uint32_t chunk_samples;   // samples of the chunk
+    uint32_t finish_paths;    // live paths the finish kernel takes once every sample is out (0: none)
     // Buffers of launch_camera_cull (null: frames it does not take): the
     // masks, and the tiles whose camera rays are traced (null: every tile).
     // With `skip_empty`, a tile without bodies and rings is not in the list:
@@ -320,10 +322,6 @@ struct AdjointWave {
 
 // Bytes of the adjoint slots for `pool` paths.
 size_t adjoint_slot_bytes(uint32_t pool);
-
-// Makes every slot of `x` free (both counters to zero: allocation j < pool
-// takes slot j); once per backward call.
-cudaError_t reset_adjoint_slots(const AdjointWave &x, uint32_t pool, cudaStream_t stream);
 
 // The samples of `p` (as launch_adjoint) through the stages; returns once
 // they have drained (host checks as launch_wavefront).

@@ -487,16 +487,45 @@ __global__ void __launch_bounds__(128) camera_cull_kernel(const __grid_constant_
     if (taken) active[at + __popc(taken_lanes & ((1u << lane) - 1u))] = tile;
 }
 
+// The list of camera_cull_kernel in raster order, by one CTA.
+__global__ void __launch_bounds__(1024) tile_list_kernel(const uint2 *masks, uint32_t *active, uint32_t *count,
+                                                         bool skip_empty, uint32_t tiles) {
+    __shared__ uint32_t warp_counts[32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t listed = 0u;
+    for (uint32_t base = 0; base < tiles; base += 1024u) {
+        const uint32_t tile = base + threadIdx.x;
+        bool taken = false;
+        if (tile < tiles) {
+            const uint2 m = masks[tile];
+            taken = !skip_empty || (m.x | m.y) != 0u;
+        }
+        const uint32_t lanes = __ballot_sync(0xffffffffu, taken);
+        if (lane == 0u) warp_counts[warp] = __popc(lanes);
+        __syncthreads();
+        uint32_t before = 0u, total = 0u;
+        for (uint32_t w = 0; w < 32u; ++w) {
+            if (w == warp) before = total;
+            total += warp_counts[w];
+        }
+        if (taken) active[listed + before + __popc(lanes & ((1u << lane) - 1u))] = tile;
+        listed += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0u) *count = listed;
+}
+
 cudaError_t launch_camera_cull(const TraceParams &p, uint2 *out, uint32_t *active, uint32_t *count, bool skip_empty,
-                               cudaStream_t stream) {
+                               bool ordered, cudaStream_t stream) {
     const uint32_t tiles_x = (p.width + kTile - 1) / kTile, tiles = tiles_x * ((p.height + kTile - 1) / kTile);
     const uint32_t n = p.s.counts[0];
     if (n == 0u || n > 32u || tiles == 0u) return cudaErrorInvalidValue;
     uint32_t group = 1u;
     while (group < n) group *= 2u;
     const uint64_t threads = (uint64_t)tiles * group;
-    camera_cull_kernel<<<(uint32_t)((threads + 127u) / 128u), 128, 0, stream>>>(p, out, active, count, skip_empty, group,
-                                                                                tiles_x, tiles);
+    camera_cull_kernel<<<(uint32_t)((threads + 127u) / 128u), 128, 0, stream>>>(p, out, ordered ? nullptr : active, count,
+                                                                                skip_empty, group, tiles_x, tiles);
+    if (ordered && active) tile_list_kernel<<<1, 1024, 0, stream>>>(out, active, count, skip_empty, tiles);
     return cudaGetLastError();
 }
 

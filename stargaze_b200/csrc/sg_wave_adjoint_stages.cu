@@ -287,8 +287,8 @@ __global__ void __launch_bounds__(kThreads, SG_WAVE_ADJ_EXTEND_MIN_BLOCKS)
     extern __shared__ float4 smem[];
     __shared__ Append<5> sm[2];
     WaveCounters *c = counters(W, t);
-    const uint32_t kept = c->cont, next = c->next;
-    const uint32_t per_sample = padded_pixels(W);
+    const uint32_t next = c->next, per_sample = padded_pixels(W);
+    const uint32_t kept = finishes(W, c, per_sample, W.finish_paths) ? 0u : c->cont;
     const uint32_t left = per_sample * W.chunk_samples - next;
     const uint32_t take = min(W.pool - kept, left);
     const uint32_t n = kept + take;
@@ -493,6 +493,7 @@ __global__ void __launch_bounds__(kShadeThreads, SG_WAVE_ADJ_SHADE_MIN_BLOCKS)
     adj_finish(const __grid_constant__ TraceParams P, const __grid_constant__ AdjointParams A,
                const __grid_constant__ WaveParams W, const __grid_constant__ AdjointWave X, uint32_t t) {
     extern __shared__ float4 smem[];
+    if (!finishes(W, counters(W, t), padded_pixels(W), W.finish_paths)) return;
     const uint32_t n = counters(W, t)->cont;
     if (blockIdx.x * kShadeThreads >= n) return;
     const BlockSink bs = open_sink(P, A, smem);

@@ -250,6 +250,15 @@ __device__ __forceinline__ uint32_t camera_tile(const WaveParams &W, uint32_t k)
     return W.active ? W.active[k] : k;
 }
 
+// The tail of a chunk: after iteration t - 1 every sample is out and at most
+// `limit` paths are left (`c` the counters of iteration t). The finish kernel
+// enqueued after it then runs them to their ends, and extend of iteration t,
+// deciding from the same counters, finds none.
+__device__ __forceinline__ bool finishes(const WaveParams &W, const WaveCounters *c, uint32_t per_sample,
+                                         uint32_t limit) {
+    return c->cont <= limit && c->next >= per_sample * W.chunk_samples;
+}
+
 // Grid of a persistent stage kernel: every resident CTA slot of every SM.
 // (Asking for the largest L1 share through the shared-memory carveout
 // halved the forward's speed and did not help the adjoint: the driver's
@@ -264,8 +273,9 @@ inline cudaError_t persistent_grid(const void *fn, size_t smem, int *grid, int t
     return cudaSuccess;
 }
 
-// Iterations the host enqueues beyond the one whose start it inspects.
-constexpr uint64_t kLookahead = 2;
+// Iterations the host enqueues beyond the one whose start it inspects (the
+// last ones find nothing to do: 1001x563 rings, 2 544, 1 527 us).
+constexpr uint64_t kLookahead = 1;
 
 // Records the end of iteration t.
 inline cudaError_t iteration_done(WaveProgress &pr, uint64_t t, cudaStream_t stream) {
@@ -287,8 +297,9 @@ inline cudaError_t started(const WaveProgress &pr, uint64_t s, WaveStart *out) {
 
 // Clears the iteration counters and the active-tile count, and culls the
 // camera rays' tiles: fills w.active_count and p.camera_cull, or clears
-// w.active and w.skip_empty where the frame is not culled.
-inline cudaError_t cull_tiles(TraceParams &p, WaveParams &w, cudaStream_t stream, WaveRun *run) {
+// w.active and w.skip_empty where the frame is not culled. `ordered`: the
+// tiles are listed in raster order.
+inline cudaError_t cull_tiles(TraceParams &p, WaveParams &w, cudaStream_t stream, WaveRun *run, bool ordered) {
     cudaError_t e = cudaMemsetAsync(w.counters, 0, (kWaveCounterSets + 1u) * sizeof(WaveCounters), stream);
     if (e != cudaSuccess) return e;
     if (!w.cull) {
@@ -297,9 +308,9 @@ inline cudaError_t cull_tiles(TraceParams &p, WaveParams &w, cudaStream_t stream
         return cudaSuccess;
     }
     w.active_count = &w.counters[kWaveCounterSets].cont;
-    if ((e = launch_camera_cull(p, w.cull, w.active, w.active_count, w.skip_empty, stream)) != cudaSuccess) return e;
+    if ((e = launch_camera_cull(p, w.cull, w.active, w.active_count, w.skip_empty, ordered, stream)) != cudaSuccess) return e;
     p.camera_cull = w.cull;
-    run->kernels += 1;
+    run->kernels += ordered ? 2 : 1;
     return cudaSuccess;
 }
 

@@ -39,8 +39,8 @@ __global__ void __launch_bounds__(kThreads, SG_WAVE_EXTEND_MIN_BLOCKS) wave_exte
     WaveCounters *c = counters(W, t);
     // Paths the previous iteration kept occupy [0, kept); new samples of the
     // chunk fill the pool up to n.
-    const uint32_t kept = c->cont, next = c->next;
-    const uint32_t per_sample = padded_pixels(W);
+    const uint32_t next = c->next, per_sample = padded_pixels(W);
+    const uint32_t kept = finishes(W, c, per_sample, W.finish_paths) ? 0u : c->cont;
     const uint32_t left = per_sample * W.chunk_samples - next;
     const uint32_t take = min(W.pool - kept, left);
     const uint32_t n = kept + take;
@@ -234,15 +234,20 @@ __global__ void __launch_bounds__(kThreads, R ? 3 : SG_WAVE_SHADE_MIN_BLOCKS) wa
 }
 
 // The tail of a chunk: once every sample is out and few paths are left,
-// stage iterations cost their launches and load chains for a handful of
-// paths each. Here every path live at the start of iteration t runs to its
-// end in its own thread through the same per-path functions (step(), as
-// the megakernel), and writes its result as the stages would.
+// stage iterations cost their launches and load chains (about 18 us) for a
+// handful of paths each. Here every path live at the start of iteration t runs
+// to its end in its own thread through the same per-path functions (step(), as
+// the megakernel), and writes its result as the stages would. Unless samples
+// are left or more than `limit` paths are live, which the GPU itself decides
+// here (and extend of iteration t alike). Its loops are as divergent as the
+// megakernel's: above a few hundred thousand paths the stages are faster
+// (launch_wavefront has the figures).
 template <bool L, bool F, bool A>
 __global__ void __launch_bounds__(kThreads, SG_WAVE_SHADE_MIN_BLOCKS) wave_finish(const __grid_constant__ TraceParams P,
                                                                             const __grid_constant__ WaveParams W,
-                                                                            uint32_t t) {
+                                                                            uint32_t t, uint32_t limit) {
     extern __shared__ float4 smem[];
+    if (!finishes(W, counters(W, t), padded_pixels(W), limit)) return;
     const uint32_t n = counters(W, t)->cont;
     if (blockIdx.x * kThreads >= n) return;
     const Scene S = stage_scene(P, smem);

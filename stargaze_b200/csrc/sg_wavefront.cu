@@ -95,11 +95,17 @@ __global__ void __launch_bounds__(kThreads) wave_resolve(const __grid_constant__
 // Host side
 // ---------------------------------------------------------------------------
 // Live paths at or below which, once every sample of the chunk is out, the
-// rest of the chunk runs in wave_finish (about one resident wave).
-#ifndef SG_WAVE_FINISH_PATHS
-#define SG_WAVE_FINISH_PATHS (1u << 18)
-#endif
-constexpr uint32_t kFinishPaths = SG_WAVE_FINISH_PATHS;
+// rest of the chunk runs in wave_finish (1080p ring dispatch: 2^17 and 2^18
+// measured alike, 2^19 and 2^20 0.5 % slower).
+constexpr uint32_t kFinishPaths = 1u << 17;
+// Samples of a chunk up to which the host enqueues a fixed number of
+// iterations and the finish kernel: one iteration up to kSingleSamples, else
+// two. Against the host loop (one, two iterations; us): three spheres 65,536
+// samples 105 (53, 78); terrain 518,819 samples 840 (676, 727); styled ring
+// scene 921,600 samples 1391 (1404, 1134); rings 3,944,941 samples 544 (1308,
+// 490); three spheres 4,194,304 samples 299 (219, 248).
+constexpr uint32_t kDirectSamples = 1u << 22;
+constexpr uint32_t kSingleSamples = 1u << 19;
 
 cudaError_t run_iteration(const WaveStages &stages, TraceParams &p, WaveParams &w, uint32_t t, const int (&grid)[4],
                           size_t smem, cudaStream_t stream, StageMarks *m) {
@@ -157,11 +163,15 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
     w.tiles_x = (p.width + kTile - 1) / kTile;
     w.tiles_y = (p.height + kTile - 1) / kTile;
     const uint32_t chunk = w.chunk_samples;
+    const uint32_t per_sample = w.tiles_x * w.tiles_y * 256u;
     // A tile whose camera rays meet no body and no ring needs no paths where a
     // ray that escapes leaves nothing: no landscape, air, sky or stored totals.
     w.skip_empty = !land && !air && !p.sky_on && !w.ck.totals;
-    if (cudaError_t e = cull_tiles(p, w, stream, run); e != cudaSuccess) return e;
-    const uint32_t per_sample = w.tiles_x * w.tiles_y * 256u;
+    // A chunk that does not fit the pool takes its tiles in a fixed order, so
+    // that the same samples share its iterations (and their tails the finish
+    // kernel) in every run.
+    const bool ordered = (uint64_t)per_sample * std::min(chunk, z) > w.pool;
+    if (cudaError_t e = cull_tiles(p, w, stream, run, ordered); e != cudaSuccess) return e;
     // A path ends within max_vertices * (bodies + 2) + 1 iterations, and an
     // iteration that takes no new sample has a full pool of paths that all
     // advance, so a chunk drains within (samples + 1) * (that + 1)
@@ -176,36 +186,46 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
         cudaError_t e = cudaSuccess;
         if (first > 0u) e = cudaMemsetAsync(w.counters, 0, kWaveCounterSets * sizeof(WaveCounters), stream);
         if (e != cudaSuccess) return e;
-        // The host reads the start of iteration t - kLookahead while the
-        // GPU runs the later ones; once one started empty the chunk has
-        // drained (the iterations after it are empty launches).
+        // A chunk that fits the pool has taken all its samples after one
+        // iteration. Up to kDirectSamples of them, the host then asks nothing:
+        // it enqueues one or two iterations and the finish kernel for whatever
+        // paths are left.
+        const bool direct = set.finish && samples <= w.pool && samples <= kDirectSamples;
+        const uint64_t direct_iterations = samples <= kSingleSamples ? 1u : 2u;
+        w.finish_paths = direct || !set.finish ? 0u : kFinishPaths;
+        // Otherwise the host reads the start of iteration t - kLookahead while
+        // the GPU runs the later ones; once one started empty the chunk has
+        // drained (the iterations after it are empty launches). The finish
+        // kernel follows every iteration that may have been the last to take
+        // samples: the GPU itself decides whether few enough paths are left
+        // (finishes()), so the tail does not wait for the host.
+        uint64_t out_by = 0;  // the first iteration after which no sample may be left
         for (uint64_t t = 0;; ++t) {
             if (t >= bound) return cudaErrorLaunchTimeout;
-            const uint32_t it = (uint32_t)t;
+            uint32_t it = (uint32_t)t;
             e = run_iteration(set, p, w, it, grid, smem, stream, marks);
             if (e != cudaSuccess) return e;
-            if ((e = iteration_done(progress, t, stream)) != cudaSuccess) return e;
-            run->iterations += 1;
             run->kernels += 3;
+            run->iterations += 1;
+            const bool last = direct && t + 1u == direct_iterations;
+            if (last || (w.finish_paths > 0u && t >= out_by)) {
+                if ((e = mark(marks, kStageFinish, stream)) != cudaSuccess) return e;
+                uint32_t next_t = it + 1u, limit = last ? samples : w.finish_paths;
+                void *args[] = {&p, &w, &next_t, &limit};
+                const uint32_t blocks = std::min<uint32_t>(grid[3], (std::min(limit, samples) + kThreads - 1) / kThreads);
+                e = cudaLaunchKernel(set.finish, dim3(blocks), dim3(kThreads), args, smem, stream);
+                if (e != cudaSuccess) return e;
+                if ((e = mark(marks, kStageGap, stream)) != cudaSuccess) return e;
+                run->kernels += 1;
+            }
+            if (last) break;
+            if (direct) continue;
+            if ((e = iteration_done(progress, t, stream)) != cudaSuccess) return e;
             if (t < kLookahead) continue;
             WaveStart start;
             if ((e = started(progress, t - kLookahead, &start)) != cudaSuccess) return e;
             if (start.kept == 0u && start.left == 0u) break;
-            // Every sample is out and few paths are left: no later iteration
-            // holds more than iteration t - kLookahead did; finish them at once.
-            if (set.finish && start.left == 0u && start.kept <= kFinishPaths) {
-                const uint32_t blocks = std::min<uint32_t>(grid[3], (start.kept + kThreads - 1) / kThreads);
-                if (blocks > 0u) {
-                    if ((e = mark(marks, kStageFinish, stream)) != cudaSuccess) return e;
-                    uint32_t next_t = it + 1u;
-                    void *args[] = {&p, &w, &next_t};
-                    e = cudaLaunchKernel(set.finish, dim3(blocks), dim3(kThreads), args, smem, stream);
-                    if (e != cudaSuccess) return e;
-                    if ((e = mark(marks, kStageGap, stream)) != cudaSuccess) return e;
-                    run->kernels += 1;
-                }
-                break;
-            }
+            out_by = start.left > 0u ? t - kLookahead + (start.left - 1u) / w.pool : 0u;
         }
         const bool first_chunk = first == 0, last_chunk = first + w.chunk_samples >= z;
         if ((e = mark(marks, kStageResolve, stream)) != cudaSuccess) return e;

@@ -104,6 +104,30 @@ __device__ __forceinline__ float2 box_interval(float3 p, float3 d, float3 extent
     return make_float2(n, f);
 }
 
+// Whether a query that has its closest hit at `t` (AU) skips a group marker's
+// box (ground.wgsl:174-181).
+static __device__ __noinline__ bool group_skipped_exact(float3 p, float3 d, float3 extent, float t) {
+    const float2 bounds = box_interval(p, d, extent);
+    return bounds.x > bounds.y || bounds.y <= 0.001f || __fdiv_rn(bounds.x, 149597870700.0f) > t;
+}
+
+// The same from the reciprocals of d, where its answer is certain: a product
+// with one differs from the quotient by less than 4e-7 of it, so do the largest
+// entry and the smallest exit, and 1e-6 decides; the few boxes closer than that
+// (and rays with a component below 1e-12, `inv.x` 0) take the six divisions.
+__device__ __forceinline__ bool group_skipped(float3 p, float3 d, float3 inv, float3 extent, float t) {
+    if (inv.x == 0.0f) return group_skipped_exact(p, d, extent, t);
+    const float ax = (-extent.x - p.x) * inv.x, bx = (extent.x - p.x) * inv.x;
+    const float ay = (-extent.y - p.y) * inv.y, by = (extent.y - p.y) * inv.y;
+    const float az = (-extent.z - p.z) * inv.z, bz = (extent.z - p.z) * inv.z;
+    const float n = fmaxf(fminf(ax, bx), fmaxf(fminf(ay, by), fminf(az, bz)));
+    const float f = fminf(fmaxf(ax, bx), fminf(fmaxf(ay, by), fmaxf(az, bz)));
+    const float far = t * 149597870700.0f, slack = 1.0e-6f * (fabsf(n) + fabsf(f));
+    if (n - f > slack || f < 0.00099f || n > far * 1.000002f) return true;
+    if (f - n > slack && f > 0.00101f && n < far * 0.999998f) return false;
+    return group_skipped_exact(p, d, extent, t);
+}
+
 // rock_hit (ground.wgsl:82-121): a box with clipped corners; 14 planes.
 static __device__ __noinline__ float4 rock_hit(float3 p, float3 d, float3 e) {
     const float3 origin = div3_rn(p, e);
@@ -535,6 +559,8 @@ static __device__ SG_HELPER LandHit landscape_query(Scene S, Counter<C, L, F> K,
     }
     const uint32_t n_objects = s->g.ground_counts[0];
     const float4 *objects = S.p->props;
+    const bool parallel = fabsf(d.x) < 1.0e-12f || fabsf(d.y) < 1.0e-12f || fabsf(d.z) < 1.0e-12f;
+    const float3 inv = parallel ? f3(0.0f, 0.0f, 0.0f) : f3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
 #pragma unroll 1
     for (uint32_t i = 0; i < n_objects; ++i) {
         const float4 oc = objects[3u * i];
@@ -544,9 +570,7 @@ static __device__ SG_HELPER LandHit landscape_query(Scene S, Counter<C, L, F> K,
         if (kind < 0.0f) {
             // Group marker: skip the subtree when its bounds are missed.
             K.add(&Events::prop_boxes);
-            const float2 bounds = box_interval(sub_rn(o, center), d, e);
-            if (bounds.x > bounds.y || bounds.y <= 0.001f || __fdiv_rn(bounds.x, kMetresPerAu) > closest.t)
-                i += (uint32_t)(-kind);
+            if (group_skipped(sub_rn(o, center), d, inv, e, closest.t)) i += (uint32_t)(-kind);
             continue;
         }
         K.add(&Events::prop_tests);

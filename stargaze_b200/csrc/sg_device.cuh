@@ -249,7 +249,7 @@ constexpr Cull kTestAll{0xffffffffu, 0xffffffffu};
 // closest_hit (pathtrace.wgsl:173-185): every body except the landscape
 // host, then the landscape.
 template <bool C, bool L, bool F>
-__device__ __forceinline__ Hit closest_hit(const Scene &S, Counter<C, L, F> K, const Ray &r, Cull cull = kTestAll) {
+__device__ __forceinline__ Hit closest_body(const Scene &S, Counter<C, L, F> K, const Ray &r, Cull cull) {
     Hit best{1.0e30f, kMiss, 0.0f, f3(0.0f, 0.0f, 0.0f)};
     const uint32_t n = S.s->counts[0];
     const float host = S.s->g.ground_north[3];
@@ -260,8 +260,13 @@ __device__ __forceinline__ Hit closest_hit(const Scene &S, Counter<C, L, F> K, c
         const float t = sphere_distance(S, K, r, i, b_radius(S, i), delta);
         if (t < best.t) best = Hit{t, i, delta, f3(0.0f, 0.0f, 0.0f)};
     }
+    return best;
+}
+template <bool C, bool L, bool F>
+__device__ __forceinline__ Hit closest_hit(const Scene &S, Counter<C, L, F> K, const Ray &r, Cull cull = kTestAll) {
+    Hit best = closest_body(S, K, r, cull);
     if constexpr (L) {
-        if (host != 0.0f) {
+        if (S.s->g.ground_north[3] != 0.0f) {
             const LandHit local = landscape_query(S, K, r, 1.0e30f, false);
             if (local.t < best.t) best = Hit{local.t, local.index, local.delta, local.n};
         }

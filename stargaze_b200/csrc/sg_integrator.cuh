@@ -168,19 +168,21 @@ struct Extension {
 // `cull`: the tile's masks for a camera ray (its first extend), else
 // kTestAll.
 template <bool C, bool L, bool F, class G>
-__device__ __forceinline__ bool extend(const Scene &S, Counter<C, L, F> K, Path &p, G &grad, Extension &e,
-                                       Cull cull = kTestAll) {
-    const sg_settings *s = S.s;
-    const uint32_t max_vertices = s->counts[3];
-    const uint32_t n_bodies = s->counts[0];
+__device__ __forceinline__ bool extend_begin(const Scene &S, Counter<C, L, F> K, Path &p, G &grad) {
+    const uint32_t max_vertices = S.s->counts[3];
+    const uint32_t n_bodies = S.s->counts[0];
     // Static bound: each of at most max_vertices vertices is preceded by at
     // most n_bodies + 1 null crossings, so valid inputs never reach it.
     if (++p.iterations > max_vertices * (n_bodies + 2u) + 1u) return false;
     if constexpr (G::adjoint) grad.iteration = p.iterations;
     K.add(&Events::vertices);
-    e.hit = closest_hit(S, K, p.ray, cull);
+    return true;
+}
+// ... from the closest hit in e.hit on.
+template <bool C, bool L, bool F, class G>
+__device__ __forceinline__ void extend_rest(const Scene &S, Counter<C, L, F> K, Path &p, G &, Extension &e, Cull cull) {
     e.disc_scale = 1.0f;
-    if (p.depth == 0u && p.null_crossings == 0u && s->background[3] > 0.0f) {
+    if (p.depth == 0u && p.null_crossings == 0u && S.s->background[3] > 0.0f) {
         const DiscHit disc = point_disc_hit(S, K, p.ray, e.hit, p.rng, cull);
         e.hit = disc.hit;
         e.disc_scale = disc.scale;
@@ -190,6 +192,13 @@ __device__ __forceinline__ bool extend(const Scene &S, Counter<C, L, F> K, Path 
     if constexpr (G::air) {
         if (S.p->air_on) air_extend(S, K, p, e.hit, e.ring);
     }
+}
+template <bool C, bool L, bool F, class G>
+__device__ __forceinline__ bool extend(const Scene &S, Counter<C, L, F> K, Path &p, G &grad, Extension &e,
+                                       Cull cull = kTestAll) {
+    if (!extend_begin(S, K, p, grad)) return false;
+    e.hit = closest_hit(S, K, p.ray, cull);
+    extend_rest(S, K, p, grad, e, cull);
     return true;
 }
 

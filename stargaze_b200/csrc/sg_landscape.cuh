@@ -501,11 +501,21 @@ static __device__ __noinline__ float4 solid_hit(float kind, float3 p, float3 v, 
     return rock_hit(p, v, e);
 }
 
+// A landscape query in its three parts: what the distant path and the host
+// sphere leave (`open`: the terrain and the primitives are still to be tested
+// from `o` along `d`), the terrain, the primitives.
+struct LandQuery {
+    LandHit closest;
+    float3 o, d;
+    bool open;
+};
+
 template <bool C, bool L, bool F>
-static __device__ SG_HELPER LandHit landscape_query(Scene S, Counter<C, L, F> K, Ray ray, float limit, bool occlusion) {
+__device__ __forceinline__ LandQuery landscape_begin(const Scene &S, Counter<C, L, F> K, const Ray &ray, float limit,
+                                                     bool occlusion) {
     LandHit closest{limit, kMiss, 0.0f, f3(0.0f, 0.0f, 0.0f)};
     const sg_settings *s = S.s;
-    if (s->g.ground_north[3] == 0.0f) return closest;
+    if (s->g.ground_north[3] == 0.0f) return {closest, f3(0.0f, 0.0f, 0.0f), f3(0.0f, 0.0f, 0.0f), false};
     const float3 o = ground_origin(S, ray);
     const float3 d = to_ground(S, ray.d);
     const float radius = s->g.ground_up[3];
@@ -514,14 +524,14 @@ static __device__ SG_HELPER LandHit landscape_query(Scene S, Counter<C, L, F> K,
         const uint32_t host = (uint32_t)s->g.ground_north[3] - 1u;
         float delta;
         const float t = sphere_distance(S, K, ray, host, b_radius(S, host), delta);
-        if (t >= 1.0e30f) return LandHit{1.0e30f, kMiss, 0.0f, f3(0.0f, 0.0f, 0.0f)};
-        return LandHit{t, host, delta, sphere_normal(S, ray, host, delta)};
+        if (t >= 1.0e30f) return {LandHit{1.0e30f, kMiss, 0.0f, f3(0.0f, 0.0f, 0.0f)}, o, d, false};
+        return {LandHit{t, host, delta, sphere_normal(S, ray, host, delta)}, o, d, false};
     }
-    if (d.y >= 0.0f && o.y > landscape_top(S)) return closest;
+    if (d.y >= 0.0f && o.y > landscape_top(S)) return {closest, o, d, false};
     if constexpr (F) {
         const LandHit host = host_sphere_fp64(S, ray, closest.t, occlusion);
         if (host.index != kMiss) {
-            if (occlusion) return host;
+            if (occlusion) return {host, o, d, false};
             closest = host;
         }
     } else {
@@ -540,7 +550,7 @@ static __device__ SG_HELPER LandHit landscape_query(Scene S, Counter<C, L, F> K,
             const float distance = t0 > 0.001f ? t0 : t1;
             const float au = __fdiv_rn(distance, kMetresPerAu);
             if (distance > 0.001f && au < closest.t) {
-                if (occlusion) return LandHit{au, kLocalBase, 0.0f, f3(0.0f, 0.0f, 0.0f)};
+                if (occlusion) return {LandHit{au, kLocalBase, 0.0f, f3(0.0f, 0.0f, 0.0f)}, o, d, false};
                 const float3 p = add_rn(o, mul_rn(d, distance));
                 const float3 n = normalize(f3(p.x / radius, 1.0f + p.y / radius, p.z / radius));
                 closest = LandHit{au, kLocalBase, 0.0f, from_ground(S, n)};
@@ -548,15 +558,28 @@ static __device__ SG_HELPER LandHit landscape_query(Scene S, Counter<C, L, F> K,
         }
     }
     }
-    if (s->g.ground_counts[1] != 0u && S.p->terrain) {
-        const float tl = __fmul_rn(fminf(closest.t, 1.0e18f), kMetresPerAu);
-        const float4 terrain = terrain_query<C>(S.p->terrain, S.p->terrain_cells, radius,
-                                                (S.s->g.ground_counts[2] & 255u) == 3u, o, d, tl, occlusion, K.ev);
-        if (terrain.w < tl && terrain.w < 1.0e29f) {
-            closest = LandHit{__fdiv_rn(terrain.w, kMetresPerAu), kTerrainId, 0.0f, from_ground(S, xyz(terrain))};
-            if (occlusion) return closest;
-        }
+    return {closest, o, d, true};
+}
+
+template <bool C, bool L, bool F>
+__device__ __forceinline__ void landscape_terrain(const Scene &S, Counter<C, L, F> K, LandQuery &q, bool occlusion) {
+    const sg_settings *s = S.s;
+    if (s->g.ground_counts[1] == 0u || !S.p->terrain) return;
+    const float tl = __fmul_rn(fminf(q.closest.t, 1.0e18f), kMetresPerAu);
+    const float4 terrain = terrain_query<C>(S.p->terrain, S.p->terrain_cells, s->g.ground_up[3],
+                                            (s->g.ground_counts[2] & 255u) == 3u, q.o, q.d, tl, occlusion, K.ev);
+    if (terrain.w < tl && terrain.w < 1.0e29f) {
+        q.closest = LandHit{__fdiv_rn(terrain.w, kMetresPerAu), kTerrainId, 0.0f, from_ground(S, xyz(terrain))};
+        if (occlusion) q.open = false;
     }
+}
+
+template <bool C, bool L, bool F>
+__device__ __forceinline__ LandHit landscape_props(const Scene &S, Counter<C, L, F> K, const LandQuery &q,
+                                                   bool occlusion) {
+    const sg_settings *s = S.s;
+    const float3 o = q.o, d = q.d;
+    LandHit closest = q.closest;
     const uint32_t n_objects = s->g.ground_counts[0];
     const float4 *objects = S.p->props;
     const bool parallel = fabsf(d.x) < 1.0e-12f || fabsf(d.y) < 1.0e-12f || fabsf(d.z) < 1.0e-12f;
@@ -625,6 +648,13 @@ static __device__ SG_HELPER LandHit landscape_query(Scene S, Counter<C, L, F> K,
         }
     }
     return closest;
+}
+
+template <bool C, bool L, bool F>
+static __device__ SG_HELPER LandHit landscape_query(Scene S, Counter<C, L, F> K, Ray ray, float limit, bool occlusion) {
+    LandQuery q = landscape_begin(S, K, ray, limit, occlusion);
+    if (q.open) landscape_terrain(S, K, q, occlusion);
+    return q.open ? landscape_props(S, K, q, occlusion) : q.closest;
 }
 
 // ---------------------------------------------------------------------------

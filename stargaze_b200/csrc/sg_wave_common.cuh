@@ -37,6 +37,9 @@ namespace {
 #endif
 constexpr int kShadeThreads = SG_WAVE_ADJ_SHADE_THREADS;
 
+// CTA size of the forward's extend stage.
+__host__ __device__ constexpr int extend_threads(bool land, bool air) { return land && air ? 512 : kThreads; }
+
 // ---------------------------------------------------------------------------
 // Path state planes
 // ---------------------------------------------------------------------------

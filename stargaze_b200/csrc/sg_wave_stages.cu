@@ -20,11 +20,21 @@ namespace {
 // ---------------------------------------------------------------------------
 // A: the host air's code and the surface styles are compiled in (frames
 // with air or styled bodies run these).
+//
+// Landscape frames under air are bound by instruction fetch (the query and the
+// air march are far larger than the instruction caches): their CTAs are of 512
+// threads and pass through the parts of an extend together. 640x360, 16
+// samples: 256 threads 6.74 ms, the same with the barriers 6.02, 512 with them
+// 5.76; 1024 without 5.83, with 6.00. The airless landscape, whose parts are
+// smaller and whose paths then live across the barriers, measured slower with
+// them (1080p, 32 samples: 47.6 against 49.2 ms) and with larger CTAs (48.5,
+// 50.5), and with smaller ones or warps that append by themselves (49.7, 53.7).
 template <bool L, bool F, bool A>
-__global__ void __launch_bounds__(kThreads, SG_WAVE_EXTEND_MIN_BLOCKS) wave_extend(const __grid_constant__ TraceParams P,
+__global__ void __launch_bounds__(extend_threads(L, A), extend_threads(L, A) == kThreads ? SG_WAVE_EXTEND_MIN_BLOCKS : 2) wave_extend(const __grid_constant__ TraceParams P,
                                                                             const __grid_constant__ WaveParams W,
                                                                             uint32_t t) {
     extern __shared__ float4 smem[];
+    constexpr int kB = extend_threads(L, A);
     // Celestial frames take several paths per append (their work per path
     // is even; SG_WAVE_EXTEND_ITEMS); landscape frames one, so that a CTA's
     // last round is small when traversal costs differ (measured with four:
@@ -35,7 +45,7 @@ __global__ void __launch_bounds__(kThreads, SG_WAVE_EXTEND_MIN_BLOCKS) wave_exte
     // from 450 to 513 ms (the barrier keeps neighbouring pixels' walks
     // through the same quadtree nodes at the same time, in L1).
     constexpr uint32_t kItems = L ? 1u : SG_WAVE_EXTEND_ITEMS;
-    __shared__ AppendK<2, kItems> sm[2];
+    __shared__ AppendK<2, kItems, kB> sm[2];
     WaveCounters *c = counters(W, t);
     // Paths the previous iteration kept occupy [0, kept); new samples of the
     // chunk fill the pool up to n.
@@ -49,27 +59,27 @@ __global__ void __launch_bounds__(kThreads, SG_WAVE_EXTEND_MIN_BLOCKS) wave_exte
         *counters(W, t + 2u) = WaveCounters{};
         W.progress[t % kProgressSlots] = make_uint2(kept, left);
     }
-    if (blockIdx.x * kThreads * kItems >= n) return;
+    if (blockIdx.x * kB * kItems >= n) return;
     const Scene S = stage_scene(P, smem);
     const Counter<false, L, F> K{nullptr};
     Forward<A> nograd;
     float4 *st = W.state[t & 1u];
     float4 *H = W.hits;
     uint32_t round = 0;
-    // Each round a thread extends kItems paths (i = base + k * kThreads +
+    // Each round a thread extends kItems paths (i = base + k * kB +
     // threadIdx.x), then the CTA appends them to the queues at once.
-    for (uint32_t base = blockIdx.x * kThreads * kItems; base < n; base += gridDim.x * kThreads * kItems, ++round) {
+    for (uint32_t base = blockIdx.x * kB * kItems; base < n; base += gridDim.x * kB * kItems, ++round) {
       uint32_t ring_bits = 0, surface_bits = 0;
 #pragma unroll 1
       for (uint32_t item = 0; item < kItems; ++item) {
-        const uint32_t i = base + item * kThreads + threadIdx.x;
+        const uint32_t i = base + item * kB + threadIdx.x;
         bool ring = false, surface = false;
-        if (i < n) {
-            Path p;
-            uint32_t slot = 0;
-            const bool fresh = i >= kept;
-            bool valid = true;
-            Cull cull = kTestAll;
+        Path p;
+        uint32_t slot = 0;
+        const bool fresh = i >= kept;
+        bool valid = i < n, was_in_air = false;
+        Cull cull = kTestAll;
+        if (valid) {
             if (fresh) {
                 // Sample k of the chunk, numbered sample-major over the
                 // padded tile grid; padding pixels are skipped.
@@ -92,48 +102,72 @@ __global__ void __launch_bounds__(kThreads, SG_WAVE_EXTEND_MIN_BLOCKS) wave_exte
             }
             // A continuation leaving the host air may be attenuated in
             // extend: it needs its throughput.
-            const bool was_in_air = A && !fresh && p.in_air;
+            was_in_air = A && !fresh && p.in_air;
             if (was_in_air) {
                 const float4 c = st[2 * W.pool + i];
                 p.throughput = xyz4(c);
                 p.previous_pdf = c.w;
             }
-            if (valid) {
-                Extension e;
-                const bool alive = extend(S, K, p, nograd, e, cull);
-                ring = alive && e.ring.index != kMiss;
-                surface = alive && !ring && e.hit.index != kMiss;
-                if (ring || surface) {
-                    if (fresh) {
-                        store_path(st, W.pool, i, p, slot);
-                    } else {
-                        st[1 * W.pool + i] = pack3u(p.ray.d, p.rng);
-                        st[6 * W.pool + i] = make_float4(iteration_word(p), depth_word(p), __uint_as_float(slot),
-                                                         __uint_as_float(p.ckpt));
-                        if (was_in_air) st[2 * W.pool + i] = pack3(p.throughput, p.previous_pdf);
-                    }
-                    if (ring) H[1 * W.pool + i] = pack3(e.ring.p, e.ring.t);
-                    else H[0 * W.pool + i] = pack3(e.hit.n, e.hit.t);
-                    H[2 * W.pool + i] = make_float4(__uint_as_float(e.hit.index), __uint_as_float(e.ring.index),
-                                                    e.hit.delta, e.disc_scale);
+        }
+        Extension e;
+        bool alive = false;
+        if constexpr (L && A) {
+            // A landscape under air: the bodies and the host sphere, the
+            // terrain, the primitives, then the air march, each by the whole
+            // CTA at a time.
+            LandQuery land;
+            land.open = false;
+            if (valid) alive = extend_begin(S, K, p, nograd);
+            if (alive) {
+                e.hit = closest_body(S, K, p.ray, cull);
+                land = landscape_begin(S, K, p.ray, 1.0e30f, false);
+            }
+            __syncthreads();
+            if (land.open) landscape_terrain(S, K, land, false);
+            __syncthreads();
+            if (land.open) land.closest = landscape_props(S, K, land, false);
+            __syncthreads();
+            if (alive) {
+                if (land.closest.t < e.hit.t)
+                    e.hit = Hit{land.closest.t, land.closest.index, land.closest.delta, land.closest.n};
+                extend_rest(S, K, p, nograd, e, cull);
+            }
+        } else {
+            if (valid) alive = extend(S, K, p, nograd, e, cull);
+        }
+        if (valid) {
+            ring = alive && e.ring.index != kMiss;
+            surface = alive && !ring && e.hit.index != kMiss;
+            if (ring || surface) {
+                if (fresh) {
+                    store_path(st, W.pool, i, p, slot);
                 } else {
-                    // Ended at the iteration bound, or escaped (then the sky
-                    // backdrop of an unscattered camera path, as
-                    // surface_vertex's miss). A new path's radiance is still
-                    // zero.
-                    if (!fresh) load_radiance_part(st, W.pool, i, p);
-                    if (alive && (P.sky_on || (A && p.sky_on_escape))) {
-                        if (!fresh && !was_in_air) p.throughput = xyz4(st[2 * W.pool + i]);
-                        // A sky-lit local surface's continuation sees the
-                        // surface sky cache (pathtrace.wgsl:1497-1499).
-                        if (A && p.sky_on_escape)
-                            p.radiance = p.radiance + p.throughput * surface_sky_lookup(S, p.ray.d);
-                        sky_miss(S, p);
-                    }
-                    W.results[slot] = finish_path(p);
-                    if (W.sky_results) W.sky_results[slot] = pack3(p.backdrop, 0.0f);
-                    if (W.ck.totals) checkpoint_total(W.ck, W.chunk_first, P.width * P.height, slot, p);
+                    st[1 * W.pool + i] = pack3u(p.ray.d, p.rng);
+                    st[6 * W.pool + i] = make_float4(iteration_word(p), depth_word(p), __uint_as_float(slot),
+                                                     __uint_as_float(p.ckpt));
+                    if (was_in_air) st[2 * W.pool + i] = pack3(p.throughput, p.previous_pdf);
                 }
+                if (ring) H[1 * W.pool + i] = pack3(e.ring.p, e.ring.t);
+                else H[0 * W.pool + i] = pack3(e.hit.n, e.hit.t);
+                H[2 * W.pool + i] = make_float4(__uint_as_float(e.hit.index), __uint_as_float(e.ring.index),
+                                                e.hit.delta, e.disc_scale);
+            } else {
+                // Ended at the iteration bound, or escaped (then the sky
+                // backdrop of an unscattered camera path, as
+                // surface_vertex's miss). A new path's radiance is still
+                // zero.
+                if (!fresh) load_radiance_part(st, W.pool, i, p);
+                if (alive && (P.sky_on || (A && p.sky_on_escape))) {
+                    if (!fresh && !was_in_air) p.throughput = xyz4(st[2 * W.pool + i]);
+                    // A sky-lit local surface's continuation sees the
+                    // surface sky cache (pathtrace.wgsl:1497-1499).
+                    if (A && p.sky_on_escape)
+                        p.radiance = p.radiance + p.throughput * surface_sky_lookup(S, p.ray.d);
+                    sky_miss(S, p);
+                }
+                W.results[slot] = finish_path(p);
+                if (W.sky_results) W.sky_results[slot] = pack3(p.backdrop, 0.0f);
+                if (W.ck.totals) checkpoint_total(W.ck, W.chunk_first, P.width * P.height, slot, p);
             }
         }
         ring_bits |= (ring ? 1u : 0u) << item;
@@ -142,10 +176,10 @@ __global__ void __launch_bounds__(kThreads, SG_WAVE_EXTEND_MIN_BLOCKS) wave_exte
       const uint32_t flags[2] = {ring_bits, surface_bits};
       uint32_t *const ctr[2] = {&c->ring, &c->surface};
       uint32_t q[2][kItems];
-      block_append_k<2, kItems>(sm[round & 1u], flags, ctr, q);
+      block_append_k<2, kItems, kB>(sm[round & 1u], flags, ctr, q);
 #pragma unroll
       for (uint32_t item = 0; item < kItems; ++item) {
-        const uint32_t i = base + item * kThreads + threadIdx.x;
+        const uint32_t i = base + item * kB + threadIdx.x;
         if ((ring_bits >> item) & 1u) W.ring_queue[q[0][item]] = i;
         if ((surface_bits >> item) & 1u) W.surface_queue[q[1][item]] = i;
       }

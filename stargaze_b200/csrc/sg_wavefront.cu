@@ -108,14 +108,14 @@ constexpr uint32_t kDirectSamples = 1u << 22;
 constexpr uint32_t kSingleSamples = 1u << 19;
 
 cudaError_t run_iteration(const WaveStages &stages, TraceParams &p, WaveParams &w, uint32_t t, const int (&grid)[4],
-                          size_t smem, cudaStream_t stream, StageMarks *m) {
+                          const int (&threads)[4], size_t smem, cudaStream_t stream, StageMarks *m) {
     void *args[] = {&p, &w, &t};
     const void *fns[3] = {stages.extend, stages.ring, stages.surface};
     const int names[3] = {kStageExtend, kStageRing, kStageSurface};
     cudaError_t e;
     for (int k = 0; k < 3; ++k) {
         if ((e = mark(m, names[k], stream)) != cudaSuccess) return e;
-        if ((e = cudaLaunchKernel(fns[k], dim3(grid[k]), dim3(kThreads), args, smem, stream)) != cudaSuccess) return e;
+        if ((e = cudaLaunchKernel(fns[k], dim3(grid[k]), dim3(threads[k]), args, smem, stream)) != cudaSuccess) return e;
     }
     return mark(m, kStageGap, stream);
 }
@@ -150,6 +150,7 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
     const size_t smem = trace_smem_bytes(p);
     const void *fns[4] = {set.extend, set.ring, set.surface, set.finish};
     int grid[4] = {0, 0, 0, 0};
+    const int threads[4] = {extend_threads(land, air), kThreads, kThreads, kThreads};
     for (int k = 0; k < 4; ++k) {
         if (!fns[k]) continue;
         const size_t bytes = smem;
@@ -157,7 +158,7 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
             cudaError_t e = cudaFuncSetAttribute(fns[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
             if (e != cudaSuccess) return e;
         }
-        cudaError_t e = persistent_grid(fns[k], bytes, &grid[k]);
+        cudaError_t e = persistent_grid(fns[k], bytes, &grid[k], threads[k]);
         if (e != cudaSuccess) return e;
     }
     w.tiles_x = (p.width + kTile - 1) / kTile;
@@ -203,7 +204,7 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
         for (uint64_t t = 0;; ++t) {
             if (t >= bound) return cudaErrorLaunchTimeout;
             uint32_t it = (uint32_t)t;
-            e = run_iteration(set, p, w, it, grid, smem, stream, marks);
+            e = run_iteration(set, p, w, it, grid, threads, smem, stream, marks);
             if (e != cudaSuccess) return e;
             run->kernels += 3;
             run->iterations += 1;

@@ -262,6 +262,31 @@ __device__ __forceinline__ bool finishes(const WaveParams &W, const WaveCounters
     return c->cont <= limit && c->next >= per_sample * W.chunk_samples;
 }
 
+// A forward stage kernel may start while its predecessor drains (launch_stage
+// with `overlap`): it stages what no kernel of the dispatch writes (bodies and
+// tables), waits for the predecessor and its memory before it reads anything
+// else, and then lets its own successor start. Every thread waits, so a kernel
+// that has completed has all its predecessors completed too.
+__device__ __forceinline__ void await_previous() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+
+inline cudaError_t launch_stage(const void *fn, uint32_t grid, uint32_t threads, void **args, size_t smem,
+                                cudaStream_t stream, bool overlap) {
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &attribute;
+    config.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelExC(&config, fn, args);
+}
+
 // Grid of a persistent stage kernel: every resident CTA slot of every SM.
 // (Asking for the largest L1 share through the shared-memory carveout
 // halved the forward's speed and did not help the adjoint: the driver's

@@ -46,6 +46,8 @@ __global__ void __launch_bounds__(extend_threads(L, A), extend_threads(L, A) == 
     // through the same quadtree nodes at the same time, in L1).
     constexpr uint32_t kItems = L ? 1u : SG_WAVE_EXTEND_ITEMS;
     __shared__ AppendK<2, kItems, kB> sm[2];
+    const Scene S = stage_scene(P, smem);
+    await_previous();
     WaveCounters *c = counters(W, t);
     // Paths the previous iteration kept occupy [0, kept); new samples of the
     // chunk fill the pool up to n.
@@ -60,7 +62,6 @@ __global__ void __launch_bounds__(extend_threads(L, A), extend_threads(L, A) == 
         W.progress[t % kProgressSlots] = make_uint2(kept, left);
     }
     if (blockIdx.x * kB * kItems >= n) return;
-    const Scene S = stage_scene(P, smem);
     const Counter<false, L, F> K{nullptr};
     Forward<A> nograd;
     float4 *st = W.state[t & 1u];
@@ -197,10 +198,11 @@ __global__ void __launch_bounds__(kThreads, R ? 3 : SG_WAVE_SHADE_MIN_BLOCKS) wa
     extern __shared__ float4 smem[];
     constexpr int kQueues = CK ? 2 : 1;
     __shared__ Append<kQueues> sm[2];
+    const Scene S = stage_scene(P, smem);
+    await_previous();
     WaveCounters *c = counters(W, t);
     const uint32_t n = R ? c->ring : c->surface;
     if (blockIdx.x * kThreads >= n) return;
-    const Scene S = stage_scene(P, smem);
     const Counter<false, L, F> K{nullptr};
     Stage<A> nograd;
     const float4 *st = W.state[t & 1u];
@@ -281,10 +283,11 @@ __global__ void __launch_bounds__(kThreads, SG_WAVE_SHADE_MIN_BLOCKS) wave_finis
                                                                             const __grid_constant__ WaveParams W,
                                                                             uint32_t t, uint32_t limit) {
     extern __shared__ float4 smem[];
+    const Scene S = stage_scene(P, smem);
+    await_previous();
     if (!finishes(W, counters(W, t), padded_pixels(W), limit)) return;
     const uint32_t n = counters(W, t)->cont;
     if (blockIdx.x * kThreads >= n) return;
-    const Scene S = stage_scene(P, smem);
     const Counter<false, L, F> K{nullptr};
     Forward<A> nograd;
     const float4 *st = W.state[t & 1u];

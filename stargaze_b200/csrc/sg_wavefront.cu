@@ -43,6 +43,7 @@ __global__ void __launch_bounds__(kThreads) wave_resolve(const __grid_constant__
                                                          const __grid_constant__ WaveParams W, int first, int last) {
     const uint32_t pixels = P.width * P.height;
     const uint32_t pixel = blockIdx.x * kThreads + threadIdx.x;
+    await_previous();
     if (pixel >= pixels) return;
     float4 total = first ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : W.totals[pixel];
     // The samples of a tile that is not traced are zero.
@@ -108,14 +109,14 @@ constexpr uint32_t kDirectSamples = 1u << 22;
 constexpr uint32_t kSingleSamples = 1u << 19;
 
 cudaError_t run_iteration(const WaveStages &stages, TraceParams &p, WaveParams &w, uint32_t t, const int (&grid)[4],
-                          const int (&threads)[4], size_t smem, cudaStream_t stream, StageMarks *m) {
+                          const int (&threads)[4], size_t smem, cudaStream_t stream, StageMarks *m, bool overlap) {
     void *args[] = {&p, &w, &t};
     const void *fns[3] = {stages.extend, stages.ring, stages.surface};
     const int names[3] = {kStageExtend, kStageRing, kStageSurface};
     cudaError_t e;
     for (int k = 0; k < 3; ++k) {
         if ((e = mark(m, names[k], stream)) != cudaSuccess) return e;
-        if ((e = cudaLaunchKernel(fns[k], dim3(grid[k]), dim3(threads[k]), args, smem, stream)) != cudaSuccess) return e;
+        if ((e = launch_stage(fns[k], grid[k], threads[k], args, smem, stream, overlap)) != cudaSuccess) return e;
     }
     return mark(m, kStageGap, stream);
 }
@@ -190,7 +191,11 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
         // A chunk that fits the pool has taken all its samples after one
         // iteration. Up to kDirectSamples of them, the host then asks nothing:
         // it enqueues one or two iterations and the finish kernel for whatever
-        // paths are left.
+        // paths are left. The finish and resolve kernels, and the stages of a
+        // single iteration, overlap their start with their predecessor's end:
+        // 256x256 spheres, 1 sample, 52.2 -> 42.6 us, rings 124 -> 117 us. The
+        // stages of larger dispatches lose by it (1001x563 rings, 7 samples,
+        // 486 -> 506 us).
         const bool direct = set.finish && samples <= w.pool && samples <= kDirectSamples;
         const uint64_t direct_iterations = samples <= kSingleSamples ? 1u : 2u;
         w.finish_paths = direct || !set.finish ? 0u : kFinishPaths;
@@ -204,7 +209,7 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
         for (uint64_t t = 0;; ++t) {
             if (t >= bound) return cudaErrorLaunchTimeout;
             uint32_t it = (uint32_t)t;
-            e = run_iteration(set, p, w, it, grid, threads, smem, stream, marks);
+            e = run_iteration(set, p, w, it, grid, threads, smem, stream, marks, direct && direct_iterations == 1u);
             if (e != cudaSuccess) return e;
             run->kernels += 3;
             run->iterations += 1;
@@ -214,7 +219,7 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
                 uint32_t next_t = it + 1u, limit = last ? samples : w.finish_paths;
                 void *args[] = {&p, &w, &next_t, &limit};
                 const uint32_t blocks = std::min<uint32_t>(grid[3], (std::min(limit, samples) + kThreads - 1) / kThreads);
-                e = cudaLaunchKernel(set.finish, dim3(blocks), dim3(kThreads), args, smem, stream);
+                e = launch_stage(set.finish, blocks, kThreads, args, smem, stream, true);
                 if (e != cudaSuccess) return e;
                 if ((e = mark(marks, kStageGap, stream)) != cudaSuccess) return e;
                 run->kernels += 1;
@@ -230,7 +235,10 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
         }
         const bool first_chunk = first == 0, last_chunk = first + w.chunk_samples >= z;
         if ((e = mark(marks, kStageResolve, stream)) != cudaSuccess) return e;
-        wave_resolve<<<(pixels + kThreads - 1) / kThreads, kThreads, 0, stream>>>(p, w, first_chunk, last_chunk);
+        int first_arg = first_chunk, last_arg = last_chunk;
+        void *args[] = {&p, &w, &first_arg, &last_arg};
+        e = launch_stage((const void *)wave_resolve, (pixels + kThreads - 1) / kThreads, kThreads, args, 0, stream, true);
+        if (e != cudaSuccess) return e;
         if ((e = mark(marks, kStageGap, stream)) != cudaSuccess) return e;
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;

@@ -37,8 +37,10 @@ namespace {
 #endif
 constexpr int kShadeThreads = SG_WAVE_ADJ_SHADE_THREADS;
 
-// CTA size of the forward's extend stage.
+// CTA sizes of the forward's extend stage and shade stages (wave_extend and
+// wave_shade say why).
 __host__ __device__ constexpr int extend_threads(bool land, bool air) { return land && air ? 512 : kThreads; }
+__host__ __device__ constexpr int shade_threads(bool land, bool ring) { return land && !ring ? 512 : kThreads; }
 
 // ---------------------------------------------------------------------------
 // Path state planes

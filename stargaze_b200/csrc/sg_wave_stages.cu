@@ -190,19 +190,24 @@ __global__ void __launch_bounds__(extend_threads(L, A), extend_threads(L, A) == 
 // Ring (R == true) or surface stage over its queue. CK: the forward stores
 // vertex checkpoints (W.ck). The ring stage runs at 3 CTAs per SM (85
 // registers, fewer spills: 13.07 → 12.81 ms per 1080p ring step; 2 CTAs
-// measured 13.57), the surface stage at 4 (3 measured slower).
+// measured 13.57), the surface stage at 4 (3 measured slower). On a landscape
+// the surface stage, bound by instruction fetch, runs in CTAs of 512 threads:
+// the append's barrier keeps twice as many warps in the same code (1080p, 32
+// samples: 14.7 ms with 256 threads, 13.3 with 512, 13.5 with 1024); celestial
+// frames, styled ones too, lose by it (styled viewer frame 0.37, 0.42, 0.48).
 template <bool L, bool F, bool R, bool A, bool CK = false>
-__global__ void __launch_bounds__(kThreads, R ? 3 : SG_WAVE_SHADE_MIN_BLOCKS) wave_shade(const __grid_constant__ TraceParams P,
+__global__ void __launch_bounds__(shade_threads(L, R), R ? 3 : SG_WAVE_SHADE_MIN_BLOCKS * kThreads / shade_threads(L, R)) wave_shade(const __grid_constant__ TraceParams P,
                                                                            const __grid_constant__ WaveParams W,
                                                                            uint32_t t) {
     extern __shared__ float4 smem[];
+    constexpr int kB = shade_threads(L, R);
     constexpr int kQueues = CK ? 2 : 1;
-    __shared__ Append<kQueues> sm[2];
+    __shared__ Append<kQueues, kB> sm[2];
     const Scene S = stage_scene(P, smem);
     await_previous();
     WaveCounters *c = counters(W, t);
     const uint32_t n = R ? c->ring : c->surface;
-    if (blockIdx.x * kThreads >= n) return;
+    if (blockIdx.x * kB >= n) return;
     const Counter<false, L, F> K{nullptr};
     Stage<A> nograd;
     const float4 *st = W.state[t & 1u];
@@ -210,7 +215,7 @@ __global__ void __launch_bounds__(kThreads, R ? 3 : SG_WAVE_SHADE_MIN_BLOCKS) wa
     const float4 *H = W.hits;
     const uint32_t *queue = R ? W.ring_queue : W.surface_queue;
     uint32_t round = 0;
-    for (uint32_t base = blockIdx.x * kThreads; base < n; base += gridDim.x * kThreads, ++round) {
+    for (uint32_t base = blockIdx.x * kB; base < n; base += gridDim.x * kB, ++round) {
         const uint32_t j = base + threadIdx.x;
         bool keep = false, record = false;
         Path p;
@@ -248,7 +253,7 @@ __global__ void __launch_bounds__(kThreads, R ? 3 : SG_WAVE_SHADE_MIN_BLOCKS) wa
             const bool flags[2] = {keep, record};
             uint32_t *const ctr[2] = {&counters(W, t + 1u)->cont, W.ck.count};
             uint32_t q[2];
-            block_append<2>(sm[round & 1u], flags, ctr, q);
+            block_append<2, kB>(sm[round & 1u], flags, ctr, q);
             if (record) {
                 if (q[1] < W.ck.capacity) {
                     p.ckpt |= 1u;
@@ -263,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, R ? 3 : SG_WAVE_SHADE_MIN_BLOCKS) wa
             const bool flags[1] = {keep};
             uint32_t *const ctr[1] = {&counters(W, t + 1u)->cont};
             uint32_t q[1];
-            block_append<1>(sm[round & 1u], flags, ctr, q);
+            block_append<1, kB>(sm[round & 1u], flags, ctr, q);
             if (keep) store_path(out, W.pool, q[0], p, slot);
         }
     }

@@ -151,7 +151,7 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
     const size_t smem = trace_smem_bytes(p);
     const void *fns[4] = {set.extend, set.ring, set.surface, set.finish};
     int grid[4] = {0, 0, 0, 0};
-    const int threads[4] = {extend_threads(land, air), kThreads, kThreads, kThreads};
+    const int threads[4] = {extend_threads(land, air), shade_threads(land, true), shade_threads(land, false), kThreads};
     for (int k = 0; k < 4; ++k) {
         if (!fns[k]) continue;
         const size_t bytes = smem;

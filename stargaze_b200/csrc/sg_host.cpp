@@ -344,19 +344,33 @@ sg_settings pack_settings(const sg_context *ctx, const sg_frame *frame, uint32_t
     return s;
 }
 
+// Copy part of a frame. A copy from pageable memory has been staged when the
+// call returns; one from pinned memory still reads it, and the caller may change
+// the frame once encode has returned, which can be before the GPU gets to the
+// copy.
+int copy_frame(sg_context *ctx, void *dst, const void *src, size_t bytes, cudaStream_t stream) {
+    SG_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream));
+    cudaPointerAttributes attributes{};
+    SG_CUDA(ctx, cudaPointerGetAttributes(&attributes, src));
+    if (attributes.type != cudaMemoryTypeUnregistered) SG_CUDA(ctx, cudaStreamSynchronize(stream));
+    return SG_OK;
+}
+
 // Write the frame's bodies and landscape primitives (src/pathtracer.rs:
 // 907-913) and refresh the terrain geometry cache when the host radius
 // changed (:933-945).
 int upload_bodies(sg_context *ctx, const sg_frame *frame, cudaStream_t stream) {
     if (frame->n_bodies)
-        SG_CUDA(ctx, cudaMemcpyAsync(ctx->bodies, frame->bodies, frame->n_bodies * sizeof(sg_sphere),
-                                     cudaMemcpyHostToDevice, stream));
+        if (int status = copy_frame(ctx, ctx->bodies, frame->bodies, frame->n_bodies * sizeof(sg_sphere), stream);
+            status != SG_OK)
+            return status;
     if (frame->globals->ground_north[3] == 0.0f) return SG_OK;
     if (frame->n_ground) {
         if (!ctx->props) SG_CUDA(ctx, cudaMalloc(&ctx->props, SG_PROP_CAPACITY * sizeof(sg_primitive)));
         if (!ctx->prop_trig) SG_CUDA(ctx, cudaMalloc(&ctx->prop_trig, SG_PROP_CAPACITY * 2 * sizeof(float4)));
-        SG_CUDA(ctx, cudaMemcpyAsync(ctx->props, frame->ground, frame->n_ground * sizeof(sg_primitive),
-                                     cudaMemcpyHostToDevice, stream));
+        if (int status = copy_frame(ctx, ctx->props, frame->ground, frame->n_ground * sizeof(sg_primitive), stream);
+            status != SG_OK)
+            return status;
         // Rotation sines and cosines per primitive (ground.wgsl:33-61): the
         // tumble angles of kind 2.25 (24 packed bits, TAU/256 steps) or the
         // yaw, each evaluated in double and rounded to f32 once per frame.

@@ -222,9 +222,10 @@ struct WaveRun {
 };
 
 // Runs the dispatch described by `p` (counts.z samples) in chunks of at
-// most w.chunk_samples samples. It reads the GPU's progress (`progress`,
-// w.progress its device ring) a few iterations behind the last one it
-// enqueued to decide whether the chunk has drained, so it returns once the
+// most w.chunk_samples samples. A small chunk that is the whole dispatch is
+// enqueued without asking the GPU anything, so the call returns at once; for a
+// larger one it reads the GPU's progress (`progress`, w.progress its device
+// ring) one iteration behind the last one it enqueued, so it returns once the
 // GPU has nearly finished. With `marks`, events bracket every stage.
 cudaError_t launch_wavefront(const TraceParams &p, WaveParams w, WaveProgress &progress, cudaStream_t stream,
                              WaveRun *run, StageMarks *marks);

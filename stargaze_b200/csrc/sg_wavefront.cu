@@ -28,7 +28,9 @@
 // megakernel does. Both integrators run the same per-path functions
 // (sg_integrator.cuh) on the same random sequences; they differ only where
 // the compiler fuses a shading multiply-add in one kernel and not in the
-// other, a few ulps. The stage kernels are in sg_wave_stages.cu.
+// other, a few ulps. Once few paths are left, finish runs each to its end in
+// its own thread; the GPU itself decides when (finishes()). The stage kernels
+// are in sg_wave_stages.cu.
 #include <algorithm>
 
 #include "sg_wave_common.cuh"

@@ -9,8 +9,9 @@ grid of `cells` cells per side (a power of two, leaves of 2x2 cells),
 
 Nodes are in breadth-first heap order: node `n` has children `4n + 1 + c`,
 child `c` covering `(x + (c & 1) * size/2, z + (c >> 1) * size/2)`; within a
-level that is Morton order. The device appends the node AABBs and vertex
-cache that `cache_terrain_geometry` computes.
+level that is Morton order. The device appends the geometry that
+`cache_terrain_geometry` computes: one record per inner node (its children's
+boxes), one per leaf (its columns, rows and curved heights) and the normals.
 
 Props (ground.wgsl:3-12, :167-240): a flat list of primitives in which a
 group marker (`center.w < 0`) bounds the next `-center.w` entries. Nesting

@@ -166,14 +166,25 @@ struct DeviceGuard {
     }
 };
 
+// Whether calls on `stream` are being recorded into a graph.
+bool recording(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(stream, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
+}
+
 // Work on `stream` comes after the last encode, also when that was on another
-// stream (encode returns with its kernels in flight).
+// stream (encode returns with its kernels in flight). Not while the stream is
+// recorded into a graph: a recording can wait for no event from outside it, an
+// event recorded into it could be waited for by nothing outside, and the graph
+// runs where its owner launches it.
 int follow_encode(sg_context *ctx, cudaStream_t stream) {
-    if (ctx->encoded && ctx->encode_stream != stream) SG_CUDA(ctx, cudaStreamWaitEvent(stream, ctx->encoded, 0));
+    if (ctx->encoded && ctx->encode_stream != stream && !recording(stream))
+        SG_CUDA(ctx, cudaStreamWaitEvent(stream, ctx->encoded, 0));
     return SG_OK;
 }
 
 int mark_encode(sg_context *ctx, cudaStream_t stream) {
+    if (recording(stream)) return SG_OK;
     if (!ctx->encoded) SG_CUDA(ctx, cudaEventCreateWithFlags(&ctx->encoded, cudaEventDisableTiming));
     SG_CUDA(ctx, cudaEventRecord(ctx->encoded, stream));
     ctx->encode_stream = stream;
@@ -347,9 +358,10 @@ sg_settings pack_settings(const sg_context *ctx, const sg_frame *frame, uint32_t
 // Copy part of a frame. A copy from pageable memory has been staged when the
 // call returns; one from pinned memory still reads it, and the caller may change
 // the frame once encode has returned, which can be before the GPU gets to the
-// copy.
+// copy. (A graph copies from the caller's memory on every launch.)
 int copy_frame(sg_context *ctx, void *dst, const void *src, size_t bytes, cudaStream_t stream) {
     SG_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream));
+    if (recording(stream)) return SG_OK;
     cudaPointerAttributes attributes{};
     SG_CUDA(ctx, cudaPointerGetAttributes(&attributes, src));
     if (attributes.type != cudaMemoryTypeUnregistered) SG_CUDA(ctx, cudaStreamSynchronize(stream));

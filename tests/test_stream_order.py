@@ -1,0 +1,71 @@
+"""Encode returns with its kernels in flight. What the caller may do then: record
+encodes into a graph, whatever stream the last encode was on and wherever the
+frame lies."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from stargaze_b200 import abi
+from stargaze_b200 import workloads as W
+from stargaze_b200._lib import check
+from stargaze_b200.pathtracer import PathTracer
+
+pytestmark = pytest.mark.gpu
+
+
+def tracer_of(wl, spp=4, integrator="wavefront", **options):
+    o = W.render_options(wl, spp, noise_seed=3)
+    for name, value in options.items():
+        setattr(o, name, value)
+    t = PathTracer((wl.width, wl.height), o)
+    W.upload_workload(t, wl)
+    t.set_integrator(integrator)
+    return t
+
+
+def encode_view(t, view, stream):
+    check(t._lib.sg_encode(t.handle, C.byref(view), C.c_void_p(stream)), t.handle)
+
+
+def pin_bodies(view):
+    """The view's bodies moved to pinned memory; returns that memory."""
+    import torch
+
+    size = view.n_bodies * C.sizeof(abi.Sphere)
+    held = torch.empty(size, dtype=torch.uint8).pin_memory()
+    C.memmove(held.data_ptr(), view.bodies, size)
+    view.bodies = C.cast(C.c_void_p(held.data_ptr()), C.POINTER(abi.Sphere))
+    return held
+
+
+@pytest.mark.parametrize("pinned", [False, True], ids=["pageable", "pinned"])
+def test_encode_records_into_a_graph(pinned):
+    """The megakernel's encode on a capturing stream that is not the last
+    encode's, then a launch of the graph: as two encodes. The image is read, and
+    a ring table uploaded, as after any encode."""
+    import torch
+
+    wl = W.rings_1080p(64, 48)
+    plain = tracer_of(wl, integrator="megakernel")
+    for _ in range(2):
+        plain.encode(wl.frame)
+    t = tracer_of(wl, integrator="megakernel")
+    view = wl.frame.view()
+    held = pin_bodies(view) if pinned else None
+    encode_view(t, view, 0)
+    torch.cuda.synchronize()
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=side):
+        encode_view(t, view, side.cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert t.samples() == plain.samples()
+    assert np.array_equal(t.read_pixels(), plain.read_pixels())
+    t.upload_ring_profile(0, wl.ring_tables[0])
+    t.encode(wl.frame)
+    assert np.isfinite(t.read_pixels()).all()
+    del held
+    graph.reset()
+    t.close()
+    plain.close()

@@ -895,8 +895,6 @@ static int meter_exposure(sg_context *ctx, cudaStream_t stream) {
         return SG_OK;
     }
     if (ctx->width == 0 || ctx->height == 0) return SG_OK;
-    DeviceGuard guard(ctx->device);
-    if (int status = follow_encode(ctx, stream); status != SG_OK) return status;
     if (!ctx->exposure) SG_CUDA(ctx, cudaMalloc(&ctx->exposure, sizeof(sg::ExposureState)));
     if (!ctx->histogram) SG_CUDA(ctx, cudaMalloc(&ctx->histogram, sg::kExposureBins * sizeof(uint32_t)));
     // Pageable source: the bytes are staged before the call returns.
@@ -994,11 +992,18 @@ static int encode_impl(sg_context *ctx, const sg_frame *frame, void *stream_ptr,
         ctx->options.sample_limit > ctx->history.samples ? ctx->options.sample_limit - ctx->history.samples : 0u;
     const uint32_t count = std::min({ctx->options.samples_per_frame, (uint32_t)SG_MAX_BATCH_SAMPLES, remaining});
     if (events) std::memset(events, 0, SG_EVENT_COUNT * sizeof(uint64_t));
-    if (count > 0 && ctx->width > 0 && ctx->height > 0) {
-        DeviceGuard guard(ctx->device);
-        const sg_settings s = pack_settings(ctx, frame, count);
+    const bool viewport = ctx->width > 0 && ctx->height > 0;
+    const bool traces = viewport && count > 0, meters = viewport && ctx->options.auto_exposure;
+    DeviceGuard guard(ctx->device);
+    // An encode with nothing to enqueue leaves the order as it was: its stream
+    // has not waited for the last one.
+    if (traces || meters) {
         status = follow_encode(ctx, stream);
-        if (status == SG_OK) status = upload_bodies(ctx, frame, stream);
+        if (status != SG_OK) return status;
+    }
+    if (traces) {
+        const sg_settings s = pack_settings(ctx, frame, count);
+        status = upload_bodies(ctx, frame, stream);
         if (status != SG_OK) return status;
         sg::TraceParams p = make_params(ctx, s);
         for (uint32_t k = 0; k < frame->n_bodies; ++k)
@@ -1083,8 +1088,7 @@ static int encode_impl(sg_context *ctx, const sg_frame *frame, void *stream_ptr,
     }
     status = meter_exposure(ctx, stream);
     if (status != SG_OK) return status;
-    {
-        DeviceGuard guard(ctx->device);
+    if (traces || meters) {
         status = mark_encode(ctx, stream);
         if (status != SG_OK) return status;
     }

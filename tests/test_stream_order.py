@@ -1,6 +1,7 @@
 """Encode returns with its kernels in flight. What the caller may do then: record
 encodes into a graph, whatever stream the last encode was on and wherever the
-frame lies."""
+frame lies; read, or upload a ring table, after encodes that had nothing to add on
+another stream."""
 import ctypes as C
 
 import numpy as np
@@ -69,3 +70,42 @@ def test_encode_records_into_a_graph(pinned):
     graph.reset()
     t.close()
     plain.close()
+
+
+def delayed_encodes(t, wl, stream):
+    """Three dispatches on `stream`, held back there for tens of milliseconds."""
+    import torch
+
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(100_000_000)
+    for _ in range(3):
+        t.encode(wl.frame, stream)
+
+
+def image_of(wl, **options):
+    t = tracer_of(wl, **options)
+    for _ in range(3):
+        t.encode(wl.frame)
+    image = t.read_pixels()
+    t.close()
+    assert np.abs(image[:, :3]).sum() > 0
+    return image
+
+
+@pytest.mark.parametrize("upload", [False, True], ids=["read", "upload"])
+def test_an_encode_with_nothing_to_add_leaves_the_order(upload):
+    """The sample limit is reached on one stream, the next encode is on another:
+    what follows there still waits for the samples."""
+    import torch
+
+    wl = W.rings_1080p(640, 360)
+    expected = image_of(wl, sample_limit=12)
+    t = tracer_of(wl, sample_limit=12)
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    delayed_encodes(t, wl, first)
+    t.encode(wl.frame, second)
+    assert t.samples() == 12
+    if upload:  # the dispatches in flight read the table they were given
+        t.upload_ring_profile(0, np.zeros(512, np.float32))
+    assert np.array_equal(t.read_pixels(second), expected)
+    t.close()

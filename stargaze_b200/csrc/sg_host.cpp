@@ -129,8 +129,7 @@ struct sg_context {
     float4 *ck_totals = nullptr;
     size_t ck_totals_size = 0;
     uint32_t *ck_count = nullptr;
-    cudaEvent_t encoded = nullptr;          // the end of the last encode, and its stream
-    cudaStream_t encode_stream = nullptr;
+    cudaEvent_t encoded = nullptr;          // the end of the last encode
     bool ck_valid = false;                  // every sample so far went through the checkpointing forward
     uint2 *camera_cull = nullptr;           // per-tile cull masks of camera rays
     size_t camera_cull_tiles = 0;
@@ -172,14 +171,15 @@ bool recording(cudaStream_t stream) {
     return cudaStreamIsCapturing(stream, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
 }
 
-// Work on `stream` comes after the last encode, also when that was on another
-// stream (encode returns with its kernels in flight). Not while the stream is
+// Work on `stream` comes after the last encode (encode returns with its kernels
+// in flight). The wait costs nothing on the same stream, and a handle does not
+// tell whether it is the same: a destroyed stream's is given out again, and
+// cudaStreamPerThread is another stream in each thread. Not while the stream is
 // recorded into a graph: a recording can wait for no event from outside it, an
 // event recorded into it could be waited for by nothing outside, and the graph
 // runs where its owner launches it.
 int follow_encode(sg_context *ctx, cudaStream_t stream) {
-    if (ctx->encoded && ctx->encode_stream != stream && !recording(stream))
-        SG_CUDA(ctx, cudaStreamWaitEvent(stream, ctx->encoded, 0));
+    if (ctx->encoded && !recording(stream)) SG_CUDA(ctx, cudaStreamWaitEvent(stream, ctx->encoded, 0));
     return SG_OK;
 }
 
@@ -187,7 +187,6 @@ int mark_encode(sg_context *ctx, cudaStream_t stream) {
     if (recording(stream)) return SG_OK;
     if (!ctx->encoded) SG_CUDA(ctx, cudaEventCreateWithFlags(&ctx->encoded, cudaEventDisableTiming));
     SG_CUDA(ctx, cudaEventRecord(ctx->encoded, stream));
-    ctx->encode_stream = stream;
     return SG_OK;
 }
 

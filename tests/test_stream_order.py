@@ -1,7 +1,7 @@
 """Encode returns with its kernels in flight. What the caller may do then: record
 encodes into a graph, whatever stream the last encode was on and wherever the
 frame lies; read, or upload a ring table, after encodes that had nothing to add on
-another stream."""
+another stream; read on a stream whose handle was the encodes'."""
 import ctypes as C
 
 import numpy as np
@@ -108,4 +108,34 @@ def test_an_encode_with_nothing_to_add_leaves_the_order(upload):
     if upload:  # the dispatches in flight read the table they were given
         t.upload_ring_profile(0, np.zeros(512, np.float32))
     assert np.array_equal(t.read_pixels(second), expected)
+    t.close()
+
+
+def test_one_handle_for_two_streams():
+    """cudaStreamPerThread in two threads: the same handle, two streams."""
+    import threading
+
+    import torch
+
+    per_thread = 2
+    wl = W.rings_1080p(640, 360)
+    plain, t = tracer_of(wl), tracer_of(wl)
+    for _ in range(4):
+        plain.encode(wl.frame)
+    t.encode(wl.frame)  # allocates
+    encoded, read = threading.Event(), threading.Event()
+
+    def encodes():
+        delayed_encodes(t, wl, torch.cuda.ExternalStream(per_thread))
+        encoded.set()
+        read.wait()
+
+    thread = threading.Thread(target=encodes)
+    thread.start()
+    encoded.wait()
+    image = t.read_pixels(per_thread)
+    read.set()
+    thread.join()
+    assert np.array_equal(image, plain.read_pixels())
+    plain.close()
     t.close()

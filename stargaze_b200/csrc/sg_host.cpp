@@ -979,28 +979,12 @@ static int camera_cull(sg_context *ctx, const sg_frame *frame, sg::TraceParams &
     return SG_OK;
 }
 
-static int encode_impl(sg_context *ctx, const sg_frame *frame, void *stream_ptr, uint64_t *events) {
-    if (!ctx) return fail(nullptr, SG_ERR_INVALID, "ctx is NULL");
-    int status = validate_frame(ctx, frame);
-    if (status != SG_OK) return status;
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-    update_history(ctx, frame);
-    // Avoid counter wrap and loss of integer resolution in f32 weights
-    // (src/pathtracer.rs:802-811).
-    const uint32_t remaining =
-        ctx->options.sample_limit > ctx->history.samples ? ctx->options.sample_limit - ctx->history.samples : 0u;
-    const uint32_t count = std::min({ctx->options.samples_per_frame, (uint32_t)SG_MAX_BATCH_SAMPLES, remaining});
-    if (events) std::memset(events, 0, SG_EVENT_COUNT * sizeof(uint64_t));
-    const bool viewport = ctx->width > 0 && ctx->height > 0;
-    const bool traces = viewport && count > 0, meters = viewport && ctx->options.auto_exposure;
-    DeviceGuard guard(ctx->device);
-    // An encode with nothing to enqueue leaves the order as it was: its stream
-    // has not waited for the last one.
-    if (traces || meters) {
-        status = follow_encode(ctx, stream);
-        if (status != SG_OK) return status;
-    }
-    if (traces) {
+// The GPU work of an encode that adds `count` samples of the viewport (none: it
+// meters only).
+static int enqueue_encode(sg_context *ctx, const sg_frame *frame, uint32_t count, cudaStream_t stream,
+                          uint64_t *events) {
+    int status = SG_OK;
+    if (count > 0) {
         const sg_settings s = pack_settings(ctx, frame, count);
         status = upload_bodies(ctx, frame, stream);
         if (status != SG_OK) return status;
@@ -1085,12 +1069,35 @@ static int encode_impl(sg_context *ctx, const sg_frame *frame, void *stream_ptr,
             for (int k = 0; k < sg::kEventCount; ++k) events[k] = host[k];
         }
     }
-    status = meter_exposure(ctx, stream);
+    return meter_exposure(ctx, stream);
+}
+
+static int encode_impl(sg_context *ctx, const sg_frame *frame, void *stream_ptr, uint64_t *events) {
+    if (!ctx) return fail(nullptr, SG_ERR_INVALID, "ctx is NULL");
+    int status = validate_frame(ctx, frame);
     if (status != SG_OK) return status;
-    if (traces || meters) {
-        status = mark_encode(ctx, stream);
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+    update_history(ctx, frame);
+    // Avoid counter wrap and loss of integer resolution in f32 weights
+    // (src/pathtracer.rs:802-811).
+    const uint32_t remaining =
+        ctx->options.sample_limit > ctx->history.samples ? ctx->options.sample_limit - ctx->history.samples : 0u;
+    const uint32_t count = std::min({ctx->options.samples_per_frame, (uint32_t)SG_MAX_BATCH_SAMPLES, remaining});
+    if (events) std::memset(events, 0, SG_EVENT_COUNT * sizeof(uint64_t));
+    const bool viewport = ctx->width > 0 && ctx->height > 0;
+    DeviceGuard guard(ctx->device);
+    // An encode with nothing to enqueue leaves the order as it was: its stream
+    // has not waited for the last one. One that fails may have enqueued a part
+    // by then, which is in flight as well.
+    const bool works = viewport && (count > 0 || ctx->options.auto_exposure);
+    if (works) {
+        status = follow_encode(ctx, stream);
         if (status != SG_OK) return status;
     }
+    status = enqueue_encode(ctx, frame, viewport ? count : 0u, stream, events);
+    const int marked = works ? mark_encode(ctx, stream) : SG_OK;
+    if (status != SG_OK) return status;
+    if (marked != SG_OK) return marked;
     ctx->history.samples += count;
     ctx->history.sequence += count;
     ctx->exposure_idle_frames = count > 0 ? 0u : (ctx->exposure_idle_frames == UINT32_MAX ? UINT32_MAX : ctx->exposure_idle_frames + 1u);

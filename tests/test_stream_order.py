@@ -1,7 +1,8 @@
 """Encode returns with its kernels in flight. What the caller may do then: record
 encodes into a graph, whatever stream the last encode was on and wherever the
 frame lies; read, or upload a ring table, after encodes that had nothing to add on
-another stream; read on a stream whose handle was the encodes'."""
+another stream; read on a stream whose handle was the encodes', or after an encode
+that failed."""
 import ctypes as C
 
 import numpy as np
@@ -9,7 +10,7 @@ import pytest
 
 from stargaze_b200 import abi
 from stargaze_b200 import workloads as W
-from stargaze_b200._lib import check
+from stargaze_b200._lib import StargazeError, check
 from stargaze_b200.pathtracer import PathTracer
 
 pytestmark = pytest.mark.gpu
@@ -138,4 +139,25 @@ def test_one_handle_for_two_streams():
     thread.join()
     assert np.array_equal(image, plain.read_pixels())
     plain.close()
+    t.close()
+
+
+def test_a_failed_encode_is_waited_for_too():
+    """An encode that fails for want of checkpoint memory has copied its frame: reading on
+    another stream comes after that copy."""
+    import torch
+
+    wl = W.rings_1080p(64, 48)
+    t = tracer_of(wl)
+    t.encode(wl.frame)
+    before = t.read_pixels()
+    t.set_checkpoints(1, 64, 1)  # a byte holds no record
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(first):
+        torch.cuda._sleep(100_000_000)
+    with pytest.raises(StargazeError) as e:
+        t.encode(wl.frame, first)
+    assert e.value.status == abi.SG_ERR_OOM
+    assert np.array_equal(t.read_pixels(second), before)
+    assert first.query()
     t.close()

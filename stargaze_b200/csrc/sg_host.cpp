@@ -71,6 +71,7 @@ struct sg_context {
     sg_primitive *props = nullptr;  // SG_PROP_CAPACITY
     float4 *prop_trig = nullptr;    // 2 float4 per prop
     std::vector<float4> trig_host;
+    std::vector<char> frame_host;   // what a frame in pinned memory is copied from
     float *terrain = nullptr;       // full layout incl. the geometry cache
     uint32_t terrain_cells = 0;
     uint32_t terrain_detail = 0;            // floats of the basalt elevation atlas
@@ -354,16 +355,22 @@ sg_settings pack_settings(const sg_context *ctx, const sg_frame *frame, uint32_t
     return s;
 }
 
-// Copy part of a frame. A copy from pageable memory has been staged when the
-// call returns; one from pinned memory still reads it, and the caller may change
-// the frame once encode has returned, which can be before the GPU gets to the
-// copy. (A graph copies from the caller's memory on every launch.)
+// Copy part of a frame. The caller may change the frame once encode has
+// returned, which can be before the GPU gets to the copy: a copy from pageable
+// memory has been staged by the driver when the call returns, and a frame in
+// pinned memory, which the copy would read later, goes through such memory of
+// the context. (A graph copies from the caller's memory on every launch.)
 int copy_frame(sg_context *ctx, void *dst, const void *src, size_t bytes, cudaStream_t stream) {
+    if (!recording(stream)) {
+        cudaPointerAttributes attributes{};
+        SG_CUDA(ctx, cudaPointerGetAttributes(&attributes, src));
+        if (attributes.type != cudaMemoryTypeUnregistered) {
+            const char *frame = static_cast<const char *>(src);
+            ctx->frame_host.assign(frame, frame + bytes);
+            src = ctx->frame_host.data();
+        }
+    }
     SG_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream));
-    if (recording(stream)) return SG_OK;
-    cudaPointerAttributes attributes{};
-    SG_CUDA(ctx, cudaPointerGetAttributes(&attributes, src));
-    if (attributes.type != cudaMemoryTypeUnregistered) SG_CUDA(ctx, cudaStreamSynchronize(stream));
     return SG_OK;
 }
 

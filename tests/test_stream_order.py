@@ -2,7 +2,7 @@
 encodes into a graph, whatever stream the last encode was on and wherever the
 frame lies; read, or upload a ring table, after encodes that had nothing to add on
 another stream; read on a stream whose handle was the encodes', or after an encode
-that failed."""
+that failed; change a frame in pinned memory."""
 import ctypes as C
 
 import numpy as np
@@ -160,4 +160,28 @@ def test_a_failed_encode_is_waited_for_too():
     assert e.value.status == abi.SG_ERR_OOM
     assert np.array_equal(t.read_pixels(second), before)
     assert first.query()
+    t.close()
+
+
+@pytest.mark.parametrize("integrator", ["megakernel", "wavefront"])
+def test_a_pinned_frame_may_change_once_encode_has_returned(integrator):
+    """And encode returns before the GPU gets to the frame's copy."""
+    import torch
+
+    wl = W.rings_1080p(64, 48)
+    plain, t = tracer_of(wl, integrator=integrator), tracer_of(wl, integrator=integrator)
+    for _ in range(2):
+        plain.encode(wl.frame)
+    t.encode(wl.frame)  # allocates
+    torch.cuda.synchronize()
+    view, stream = wl.frame.view(), torch.cuda.Stream()
+    held = pin_bodies(view)
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(200_000_000)
+    asleep = stream.record_event()
+    encode_view(t, view, stream.cuda_stream)
+    assert not asleep.query()
+    held.zero_()
+    assert np.array_equal(t.read_pixels(stream), plain.read_pixels())
+    plain.close()
     t.close()

@@ -996,8 +996,12 @@ static int enqueue_encode(sg_context *ctx, const sg_frame *frame, uint32_t count
         status = upload_bodies(ctx, frame, stream);
         if (status != SG_OK) return status;
         sg::TraceParams p = make_params(ctx, s);
-        for (uint32_t k = 0; k < frame->n_bodies; ++k)
-            if (frame->bodies[k].axis_x[3] >= 0.5f) p.styled = 1u;
+        bool ringed = false;
+        for (uint32_t k = 0; k < frame->n_bodies; ++k) {
+            const sg_sphere &b = frame->bodies[k];
+            if (b.axis_x[3] >= 0.5f) p.styled = 1u;
+            if (b.ring_params[0] > b.ring_plane[3] && b.ring_params[1] > 0.0f) ringed = true;
+        }
         // A backdrop left by an earlier sky (the history has reset since).
         if (!p.sky_on && ctx->backdrop_written) {
             SG_CUDA(ctx, cudaMemsetAsync(ctx->backdrop, 0, (size_t)ctx->width * ctx->height * sizeof(float4), stream));
@@ -1030,6 +1034,7 @@ static int enqueue_encode(sg_context *ctx, const sg_frame *frame, uint32_t count
             status = ensure_wave(ctx, count, w);
             if (status == SG_OK) status = ensure_cull(ctx, frame, &w.cull, &w.active, stream);
             if (status != SG_OK) return status;
+            w.long_tails = ringed || p.styled;
             if (ctx->ck_valid) {
                 status = ensure_checkpoints(ctx, stream);
                 if (status != SG_OK) return status;

@@ -170,6 +170,7 @@ struct WaveParams {
     uint32_t chunk_first;     // first sample of the chunk within the dispatch
     uint32_t chunk_samples;   // samples of the chunk
     uint32_t finish_paths;    // live paths the finish kernel takes once every sample is out (0: none)
+    bool long_tails;          // a body has a ring (paths cross it) or a procedural surface (dear to shade)
     // Buffers of launch_camera_cull (null: frames it does not take): the
     // masks, and the tiles whose camera rays are traced (null: every tile).
     // With `skip_empty`, a tile without bodies and rings is not in the list:

@@ -102,13 +102,30 @@ __global__ void __launch_bounds__(kThreads) wave_resolve(const __grid_constant__
 // measured alike, 2^19 and 2^20 0.5 % slower).
 constexpr uint32_t kFinishPaths = 1u << 17;
 // Samples of a chunk up to which the host enqueues a fixed number of
-// iterations and the finish kernel: one iteration up to kSingleSamples, else
-// two. Against the host loop (one, two iterations; us): three spheres 65,536
-// samples 105 (53, 78); terrain 518,819 samples 840 (676, 727); styled ring
-// scene 921,600 samples 1391 (1404, 1134); rings 3,944,941 samples 544 (1308,
-// 490); three spheres 4,194,304 samples 299 (219, 248).
+// iterations and the finish kernel for every path left: one iteration up to
+// kSingleSamples, else two. How many paths that leaves depends on the view, which
+// the host does not know, so the rule has to hold where every camera ray meets
+// something, too. Celestial frames with rings or procedural surfaces keep more
+// and dearer paths: there one iteration only up to kSingleLongTails, and with
+// surfaces a third one above kTwoStyled, which finds nothing where the paths after
+// the second were at most kFewPaths: the finish kernel has taken them then. (Plain
+// rings go without: it would cost every wide view 8 us.) Above kDirectSamples the
+// host asks.
+// Eight bounces, us, the host loop | one iteration | two | three ("narrow": a
+// tenth to a third of the field, where most rays meet something):
+//                              2^18 samples          2^19             2^22
+//   three spheres                    -        120 |  57 |  89    274 | - |  243
+//   rings                      - | 166 | 172  240 | 262 | 208    735 | - |  679 |  693
+//   rings, narrow              - | 235 | 198  311 | 443 | 279   1388 | - | 1579 | 1370
+//   styled rings               - | 460 | 444  601 | 715 | 569   2264 | - | 2096 | 2107
+//   styled rings, narrow       - | 485 | 550  765 | 813 | 730   2931 | - | 3389 | 2968
+//   terrain                          -        618 | 476 | 497   2299 | - | 2213
+//   terrain, narrow                  -        706 | 663 | 595   2717 | - | 2629
 constexpr uint32_t kDirectSamples = 1u << 22;
 constexpr uint32_t kSingleSamples = 1u << 19;
+constexpr uint32_t kSingleLongTails = 1u << 18;
+constexpr uint32_t kTwoStyled = 1u << 21;
+constexpr uint32_t kFewPaths = 1u << 18;
 
 cudaError_t run_iteration(const WaveStages &stages, TraceParams &p, WaveParams &w, uint32_t t, const int (&grid)[4],
                           const int (&threads)[4], size_t smem, cudaStream_t stream, StageMarks *m, bool overlap) {
@@ -192,14 +209,16 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
         if (e != cudaSuccess) return e;
         // A chunk that fits the pool has taken all its samples after one
         // iteration. Up to kDirectSamples of them, the host then asks nothing:
-        // it enqueues one or two iterations and the finish kernel for whatever
+        // it enqueues one to three iterations and the finish kernel for whatever
         // paths are left. The finish and resolve kernels, and the stages of a
-        // single iteration, overlap their start with their predecessor's end:
+        // single iteration or a third, overlap their start with their predecessor's end:
         // 256x256 spheres, 1 sample, 52.2 -> 42.6 us, rings 124 -> 117 us. The
         // stages of larger dispatches lose by it (1001x563 rings, 7 samples,
         // 486 -> 506 us).
         const bool direct = set.finish && samples <= w.pool && samples <= kDirectSamples;
-        const uint64_t direct_iterations = samples <= kSingleSamples ? 1u : 2u;
+        const uint32_t single = w.long_tails && !land ? kSingleLongTails : kSingleSamples;
+        const bool third = p.styled && !land && samples > kTwoStyled;
+        const uint64_t direct_iterations = samples <= single ? 1u : third ? 3u : 2u;
         w.finish_paths = direct || !set.finish ? 0u : kFinishPaths;
         // Otherwise the host reads the start of iteration t - kLookahead while
         // the GPU runs the later ones; once one started empty the chunk has
@@ -211,14 +230,17 @@ cudaError_t launch_wavefront(const TraceParams &params, WaveParams w, WaveProgre
         for (uint64_t t = 0;; ++t) {
             if (t >= bound) return cudaErrorLaunchTimeout;
             uint32_t it = (uint32_t)t;
-            e = run_iteration(set, p, w, it, grid, threads, smem, stream, marks, direct && direct_iterations == 1u);
+            if (direct) w.finish_paths = t == 2u ? kFewPaths : 0u;  // what finish was given before iteration t
+            e = run_iteration(set, p, w, it, grid, threads, smem, stream, marks,
+                              direct && (direct_iterations == 1u || t == 2u));
             if (e != cudaSuccess) return e;
             run->kernels += 3;
             run->iterations += 1;
             const bool last = direct && t + 1u == direct_iterations;
-            if (last || (w.finish_paths > 0u && t >= out_by)) {
+            const bool few = direct && !last && t == 1u;
+            if (last || few || (!direct && w.finish_paths > 0u && t >= out_by)) {
                 if ((e = mark(marks, kStageFinish, stream)) != cudaSuccess) return e;
-                uint32_t next_t = it + 1u, limit = last ? samples : w.finish_paths;
+                uint32_t next_t = it + 1u, limit = last ? samples : few ? kFewPaths : w.finish_paths;
                 void *args[] = {&p, &w, &next_t, &limit};
                 const uint32_t blocks = std::min<uint32_t>(grid[3], (std::min(limit, samples) + kThreads - 1) / kThreads);
                 e = launch_stage(set.finish, blocks, kThreads, args, smem, stream, true);

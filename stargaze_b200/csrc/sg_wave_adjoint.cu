@@ -8,10 +8,19 @@ namespace sg {
 
 namespace {
 
-// Live paths at or below which, once every sample is out, the rest of the
-// replay runs in adj_finish. Ring scene, 512x512, 64 samples, render and
-// gradient: 2^14 8.47, 2^16 8.37, 2^17 8.82, 2^18 9.82 ms.
+// When the rest of the replay runs in adj_finish. On a landscape, and where that
+// holds for all samples after the first iteration: once every sample is out and
+// at most kFinishPaths paths are left, which the GPU itself decides (finishes()).
+// In celestial frames such paths are mostly second replays with most of their
+// length to go, and the finish kernel, divergent, is slower with tens of
+// thousands of them than the stages: there it waits until the host has seen an
+// iteration start with at most kSeenPaths, and one more has run. Backward alone,
+// eight bounces, us; ring scene: 333x217, 7 samples, 909 (1017 when the GPU decided
+// at 2^16), 1024x1024, 2 samples, 1479 (2110), 512x512, 16 samples, 2154 (2792), 64
+// samples, 5692 (5756); with two bounces, whose replays are short, 512x512, 4
+// samples, 759 (720). Terrain, 512x512, 4 samples: 1519 as it is, 1614 by the host.
 constexpr uint32_t kFinishPaths = 1u << 16;
+constexpr uint32_t kSeenPaths = 1u << 17;
 
 }  // namespace
 
@@ -60,12 +69,24 @@ cudaError_t launch_adjoint_wavefront(const TraceParams &params, const AdjointPar
     const uint64_t bound = ((uint64_t)samples + 1u) * cap;
     // A tile whose camera rays meet nothing has no gradient.
     w.skip_empty = !land;
-    w.finish_paths = kFinishPaths;
+    const bool whole = samples <= kFinishPaths && samples <= w.pool;
+    const bool device_decides = land || whole;
+    w.finish_paths = device_decides ? kFinishPaths : 0u;
     cudaError_t e = cull_tiles(p, w, stream, run, false);
     if (e != cudaSuccess) return e;
     // Every slot is free (both counters zero: allocation j < pool takes slot
     // j); the finish kernel of an earlier launch gave none of its slots back.
     if ((e = cudaMemsetAsync(x.free_ends, 0, 2 * sizeof(uint32_t), stream)) != cudaSuccess) return e;
+    // The finish kernel for the paths live at the start of iteration t, if they
+    // are at most `limit`.
+    auto finish = [&](uint32_t t, uint32_t limit, uint32_t most) -> cudaError_t {
+        WaveParams taken = w;
+        taken.finish_paths = limit;
+        void *args[] = {&p, &a, &taken, &x, &t};
+        const uint32_t blocks = std::min<uint32_t>(grid[3], (std::min(most, samples) + kShadeThreads - 1) / kShadeThreads);
+        run->kernels += 1;
+        return cudaLaunchKernel(set.finish, dim3(blocks), dim3(kShadeThreads), args, smem[1], stream);
+    };
     uint64_t out_by = 0;  // as in launch_wavefront
     for (uint64_t t = 0;; ++t) {
         if (t >= bound) return cudaErrorLaunchTimeout;
@@ -77,22 +98,19 @@ cudaError_t launch_adjoint_wavefront(const TraceParams &params, const AdjointPar
             if (e != cudaSuccess) return e;
         }
         run->kernels += 3;
-        if (t >= out_by) {
-            uint32_t next_t = it + 1u;
-            void *last[] = {&p, &a, &w, &x, &next_t};
-            const uint32_t blocks =
-                std::min<uint32_t>(grid[3], (std::min(w.finish_paths, samples) + kShadeThreads - 1) / kShadeThreads);
-            e = cudaLaunchKernel(set.finish, dim3(blocks), dim3(kShadeThreads), last, smem[1], stream);
-            if (e != cudaSuccess) return e;
-            run->kernels += 1;
-        }
         run->iterations += 1;
-        if (samples <= w.finish_paths && samples <= w.pool) break;
+        if (device_decides && t >= out_by && (e = finish(it + 1u, kFinishPaths, kFinishPaths)) != cudaSuccess) return e;
+        if (whole) break;
         if ((e = iteration_done(progress, t, stream)) != cudaSuccess) return e;
         if (t < kLookahead) continue;
         WaveStart start;
         if ((e = started(progress, t - kLookahead, &start)) != cudaSuccess) return e;
         if (start.kept == 0u && start.left == 0u) break;
+        if (!device_decides && start.left == 0u && start.kept <= kSeenPaths) {
+            // Every sample is out, and no later iteration holds more paths.
+            if ((e = finish(it + 1u, samples, start.kept)) != cudaSuccess) return e;
+            break;
+        }
         out_by = start.left > 0u ? t - kLookahead + (start.left - 1u) / w.pool : 0u;
     }
     return cudaSuccess;

@@ -204,8 +204,23 @@ SG_API int sg_get_options(const sg_context *ctx, sg_options *options);
 
 /* PathTracer::encode (src/pathtracer.rs:789-1009): validate capacities,
  * update the history, clamp the batch to SG_MAX_BATCH_SAMPLES and the
- * sample limit, upload the frame and enqueue the trace kernel on `stream`.
- * The call returns once the work is enqueued. */
+ * sample limit, upload the frame and enqueue the trace kernels on `stream`.
+ *
+ * The call returns with that work in flight (the wavefront integrator's larger
+ * dispatches: with the rest of it, see sg_set_integrator); an error of a kernel
+ * may show in a later call. The frame may change as soon as the call has
+ * returned, wherever it lies.
+ * Other calls on the context, on whichever stream, come after the last encode:
+ * reads, display, metering, queries, sg_backward and encodes wait for it on the
+ * GPU, the uploads and sg_get_checkpoint_stats on the host. Nothing waits for
+ * a display into device memory, which is in flight too when it returns. A
+ * caller's own kernels and copies that use the pointer of
+ * sg_accumulation_device_ptr have to be on the last encode's stream or to wait
+ * for it.
+ * On a capturing stream the work is recorded into the graph; the context's
+ * buffers have to be there (encode once before), and each launch of the graph
+ * copies the frame from where it was. Nothing of the above orders the graph's
+ * launches: the caller does. */
 SG_API int sg_encode(sg_context *ctx, const sg_frame *frame, void *stream);
 
 /* History counters (PathTracer::samples, src/pathtracer.rs:742-744;
@@ -235,7 +250,8 @@ SG_API int sg_set_accumulation(sg_context *ctx, const float *src, int src_on_dev
                         uint32_t samples, uint32_t sequence, void *stream);
 
 /* Device pointer of the accumulation (width*height float4), valid until the
- * next sg_resize / sg_destroy. */
+ * next sg_resize / sg_destroy. Work of the caller's on it is not ordered after
+ * the encodes (see sg_encode). */
 SG_API int sg_accumulation_device_ptr(sg_context *ctx, void **ptr);
 
 /* ------------------------------------------------------------------ */
@@ -408,10 +424,14 @@ SG_API int sg_get_checkpoint_stats(sg_context *ctx, uint64_t *device_bytes, uint
  * accumulations agree to a few ulps (the compiler fuses shading multiply-
  * adds differently in the two kernels). The wavefront allocates its pool
  * and a per-sample radiance buffer (16 B per pixel and sample, up to
- * 2.25 GiB; larger dispatches run in sample chunks) on first use, and its
- * sg_encode returns once the dispatch's stages have drained (it reads a
- * 32-byte counter back every few iterations). sg_encode_counted always runs
- * the megakernel. The choice does not reset the accumulation. */
+ * 2.25 GiB; larger dispatches run in sample chunks) on first use. Its
+ * sg_encode follows the stages of a chunk of more than 2^22 samples (pixels
+ * padded to 16x16 tiles), of one larger than the pool and of one that stores
+ * checkpoint records, through a counter in host memory, and returns when they
+ * have nearly drained (not on a capturing stream, which cannot be waited
+ * for); smaller dispatches are enqueued whole and in flight when it returns.
+ * sg_encode_counted always runs the megakernel. The choice does not reset the
+ * accumulation. */
 #define SG_INTEGRATOR_MEGAKERNEL 0
 #define SG_INTEGRATOR_WAVEFRONT 1
 #define SG_WAVE_MAX_POOL (1u << 26)

@@ -223,11 +223,12 @@ struct WaveRun {
 };
 
 // Runs the dispatch described by `p` (counts.z samples) in chunks of at
-// most w.chunk_samples samples. A small chunk that is the whole dispatch is
-// enqueued without asking the GPU anything, so the call returns at once; for a
-// larger one it reads the GPU's progress (`progress`, w.progress its device
-// ring) one iteration behind the last one it enqueued, so it returns once the
-// GPU has nearly finished. With `marks`, events bracket every stage.
+// most w.chunk_samples samples. A chunk of at most 2^22 samples that fits the
+// pool (without checkpoint records) is enqueued without asking the GPU anything;
+// for others the host reads the GPU's progress (`progress`, w.progress its device
+// ring) one iteration behind the last one it enqueued, so that it goes on once the
+// GPU has nearly finished the chunk. The call returns with its last chunk's work
+// in flight. With `marks`, events bracket every stage.
 cudaError_t launch_wavefront(const TraceParams &p, WaveParams w, WaveProgress &progress, cudaStream_t stream,
                              WaveRun *run, StageMarks *marks);
 cudaError_t launch_closest_hit(const TraceParams &p, const sg_ray *rays, sg_hit *hits, uint32_t n,

@@ -37,10 +37,16 @@ namespace {
 #endif
 constexpr int kShadeThreads = SG_WAVE_ADJ_SHADE_THREADS;
 
-// CTA sizes of the forward's extend stage and shade stages (wave_extend and
-// wave_shade say why).
+// CTA sizes of the forward's extend stage and shade stages, and the CTAs per SM
+// they are compiled for (wave_extend and wave_shade say why).
 __host__ __device__ constexpr int extend_threads(bool land, bool air) { return land && air ? 512 : kThreads; }
+__host__ __device__ constexpr int extend_blocks(bool land, bool air) {
+    return land && air ? 2 : SG_WAVE_EXTEND_MIN_BLOCKS;
+}
 __host__ __device__ constexpr int shade_threads(bool land, bool ring) { return land && !ring ? 512 : kThreads; }
+__host__ __device__ constexpr int shade_blocks(bool land, bool ring) {
+    return ring ? 3 : SG_WAVE_SHADE_MIN_BLOCKS * kThreads / shade_threads(land, ring);
+}
 
 // ---------------------------------------------------------------------------
 // Path state planes

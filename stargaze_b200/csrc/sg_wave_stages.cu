@@ -30,9 +30,8 @@ namespace {
 // them (1080p, 32 samples: 47.6 against 49.2 ms) and with larger CTAs (48.5,
 // 50.5), and with smaller ones or warps that append by themselves (49.7, 53.7).
 template <bool L, bool F, bool A>
-__global__ void __launch_bounds__(extend_threads(L, A), extend_threads(L, A) == kThreads ? SG_WAVE_EXTEND_MIN_BLOCKS : 2) wave_extend(const __grid_constant__ TraceParams P,
-                                                                            const __grid_constant__ WaveParams W,
-                                                                            uint32_t t) {
+__global__ void __launch_bounds__(extend_threads(L, A), extend_blocks(L, A))
+    wave_extend(const __grid_constant__ TraceParams P, const __grid_constant__ WaveParams W, uint32_t t) {
     extern __shared__ float4 smem[];
     constexpr int kB = extend_threads(L, A);
     // Celestial frames take several paths per append (their work per path
@@ -196,9 +195,8 @@ __global__ void __launch_bounds__(extend_threads(L, A), extend_threads(L, A) == 
 // samples: 14.7 ms with 256 threads, 13.3 with 512, 13.5 with 1024); celestial
 // frames, styled ones too, lose by it (styled viewer frame 0.37, 0.42, 0.48).
 template <bool L, bool F, bool R, bool A, bool CK = false>
-__global__ void __launch_bounds__(shade_threads(L, R), R ? 3 : SG_WAVE_SHADE_MIN_BLOCKS * kThreads / shade_threads(L, R)) wave_shade(const __grid_constant__ TraceParams P,
-                                                                           const __grid_constant__ WaveParams W,
-                                                                           uint32_t t) {
+__global__ void __launch_bounds__(shade_threads(L, R), shade_blocks(L, R))
+    wave_shade(const __grid_constant__ TraceParams P, const __grid_constant__ WaveParams W, uint32_t t) {
     extern __shared__ float4 smem[];
     constexpr int kB = shade_threads(L, R);
     constexpr int kQueues = CK ? 2 : 1;

@@ -78,13 +78,13 @@ OPS_PER_EVENT = {
 EVENT_ORDER = ["vertices", "sphere_tests", "sphere_hits", "ring_tests", "light_samples", "shadow_rays",
                "ring_events", "surface_events", "rng_draws", "terrain_nodes", "terrain_triangles", "prop_boxes",
                "prop_tests"]
-# DRAM traffic of one 64-sample dispatch of the ring workload: an ncu
-# capture of one steady-state iteration of the three stage kernels (4 Mi-path
-# pool: 655 MB for 4.19 M path extensions) scaled to the dispatch's 183 M
-# path extensions (1.38 per sample, counting kernel). Issue-slot fraction of
-# the same capture, weighted by the stages' share of the step.
-TRAFFIC_BYTES_PER_LAUNCH = 654.6e6 * (1.38 * 1920 * 1080 * 64) / 4.194e6
-ISSUE_SLOT_FRACTION = 0.60
+# DRAM traffic of one 64-sample dispatch of the ring workload: the sum over
+# every launch of one dispatch under ncu (4 Mi-path pool: 16.15 GB read, 12.10
+# written). Issue-slot fraction: a capture of one steady-state iteration of the
+# three stage kernels (71, 60 and 53 %), weighted by their share of the step.
+# Both in profiles/wavefront_rings_1080p_instruction_mix.md.
+TRAFFIC_BYTES_PER_LAUNCH = 28.25e9
+ISSUE_SLOT_FRACTION = 0.61
 L2_FLUSH_BYTES = 256 << 20
 
 
@@ -866,7 +866,9 @@ def run_ours(args):
     # Queue and result traffic by construction (wavefront): an extension
     # reads 3 and writes 4 float4 (planes 0, 1, 6; planes 1, 6 and two hit
     # planes), a shade vertex reads 7 planes and 2 hit planes and writes 7
-    # planes, every sample writes and the resolve reads one float4.
+    # planes, every sample writes and the resolve reads one float4. (An upper
+    # bound: camera rays of tiles that meet nothing, and new paths that escape
+    # at once, are counted although they move no planes.)
     ev = {n: int(totals[k]) / batches for k, n in enumerate(EVENT_ORDER)}
     queue_bytes = (ev["vertices"] * 7 + (ev["ring_events"] + ev["surface_events"]) * 16) * 16 + \
         wl.width * wl.height * BATCH * 32
@@ -914,7 +916,7 @@ def run_ours(args):
             "roofline": {"bound": "fp32", "achieved": achieved / 1e12, "peak": peak.value / 1e12, "unit": "TFLOP/s",
                          "frac": achieved / peak.value,
                          "traffic": TRAFFIC_BYTES_PER_LAUNCH if wl.name == "rings_1080p" else None,
-                         "traffic_note": "scaled from a one-iteration capture by path extensions",
+                         "traffic_note": "sum over the launches of one dispatch, ncu, 4 Mi-path pool",
                          "algorithmic_bytes_per_launch": queue_bytes,
                          "queue_hbm_frac": queue_bytes / (statistics.mean(launch_ms) * 1e-3) / (hbm_peak_gbs * 1e9)
                          if hbm_peak_gbs else None,

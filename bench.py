@@ -82,7 +82,6 @@ EVENT_ORDER = ["vertices", "sphere_tests", "sphere_hits", "ring_tests", "light_s
 # every launch of one dispatch under ncu (4 Mi-path pool: 16.15 GB read, 12.10
 # written). Issue-slot fraction: a capture of one steady-state iteration of the
 # three stage kernels (71, 60 and 53 %), weighted by their share of the step.
-# Both in profiles/wavefront_rings_1080p_instruction_mix.md.
 TRAFFIC_BYTES_PER_LAUNCH = 28.25e9
 ISSUE_SLOT_FRACTION = 0.61
 L2_FLUSH_BYTES = 256 << 20

@@ -1097,19 +1097,20 @@ static int encode_impl(sg_context *ctx, const sg_frame *frame, void *stream_ptr,
     const uint32_t count = std::min({ctx->options.samples_per_frame, (uint32_t)SG_MAX_BATCH_SAMPLES, remaining});
     if (events) std::memset(events, 0, SG_EVENT_COUNT * sizeof(uint64_t));
     const bool viewport = ctx->width > 0 && ctx->height > 0;
-    DeviceGuard guard(ctx->device);
     // An encode with nothing to enqueue leaves the order as it was: its stream
     // has not waited for the last one. One that fails may have enqueued a part
     // by then, which is in flight as well.
-    const bool works = viewport && (count > 0 || ctx->options.auto_exposure);
-    if (works) {
+    if (viewport && (count > 0 || ctx->options.auto_exposure)) {
+        DeviceGuard guard(ctx->device);
         status = follow_encode(ctx, stream);
         if (status != SG_OK) return status;
+        status = enqueue_encode(ctx, frame, count, stream, events);
+        const int marked = mark_encode(ctx, stream);
+        if (status == SG_OK) status = marked;
+    } else {
+        status = meter_exposure(ctx, stream);
     }
-    status = enqueue_encode(ctx, frame, viewport ? count : 0u, stream, events);
-    const int marked = works ? mark_encode(ctx, stream) : SG_OK;
     if (status != SG_OK) return status;
-    if (marked != SG_OK) return marked;
     ctx->history.samples += count;
     ctx->history.sequence += count;
     ctx->exposure_idle_frames = count > 0 ? 0u : (ctx->exposure_idle_frames == UINT32_MAX ? UINT32_MAX : ctx->exposure_idle_frames + 1u);
